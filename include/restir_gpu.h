@@ -63,8 +63,8 @@ extern "C" {
 #define RESTIR_TRACE_ANY 1               /* stackless, first hit (bvh.sh:140-174) */
 #define RESTIR_TRACE_CLOSEST_STACKLESS 2 /* stackless, nearest hit (bvh.sh:140-174) */
 #define RESTIR_TRACE_CLOSEST_WATERTIGHT 3 /* full stack, watertight triangle test */
-#define RESTIR_TRACE_CLOSEST_QUEUE 4     /* RESTIR_TRACE_CLOSEST through the persistent
-                                            queue tracer (same results; no reference
+#define RESTIR_TRACE_CLOSEST_QUEUE 4     /* RESTIR_TRACE_CLOSEST through the queue
+                                            tracer's loop (same results; no reference
                                             counterpart) */
 #define RESTIR_TRACE_ANY_WAVE 5          /* any hit in warp lock step (bvh.sh:177-212); rays
                                             32i..32i+31 form one warp */

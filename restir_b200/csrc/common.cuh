@@ -260,7 +260,10 @@ __device__ __forceinline__ void countWork(int kind, uint32_t nodes, uint32_t tri
 	const unsigned t = __reduce_add_sync(mask, triangles);
 	if (int(threadIdx.x & 31u) == __ffs(mask) - 1)
 	{
-		atomicAdd(&g_restirCounters[kind], static_cast<unsigned long long>(__popc(mask)));
+		if (kind >= 0) // -1: a ray counted before
+		{
+			atomicAdd(&g_restirCounters[kind], static_cast<unsigned long long>(__popc(mask)));
+		}
 		atomicAdd(&g_restirCounters[kind == RESTIR_COUNT_SCREEN ? RESTIR_COUNT_SCREEN_STEPS : RESTIR_COUNT_NODES],
 			static_cast<unsigned long long>(n));
 		if (kind != RESTIR_COUNT_SCREEN)

@@ -543,18 +543,27 @@ __global__ void __launch_bounds__(kGiThreads, RESTIR_GI_CANDIDATES_MIN_BLOCKS) g
 	}
 }
 
-__global__ void __launch_bounds__(128) traceQueueKernel(BvhView bvh, RayQueue queue)
+// The queue tracers (wavefront.cuh): nearest hits in two launches for the GI
+// candidates and the cache's training, the stackless walk for the specular rays.
+template<bool kWide, int kThreads>
+__global__ void __launch_bounds__(kThreads, 1024 / kThreads) traceQueueKernel(BvhView bvh, RayQueue queue)
 {
-	__shared__ int stackStorage[kBvhShortStack * 128];
-	traceQueueClosest<128>(bvh, queue, stackStorage);
+	__shared__ NearestStorage storage[kThreads / 32];
+	queueNearest<kWide>(bvh, queue, storage);
 }
 
-// The queue tracer at other block sizes (restir_trace_queue's tuning knob).
-template<int kThreads>
-__global__ void __launch_bounds__(kThreads) traceQueueSizedKernel(BvhView bvh, RayQueue queue)
+template<bool kWide, int kThreads>
+__global__ void __launch_bounds__(kThreads, 1024 / kThreads) rewalkQueueKernel(BvhView bvh, RayQueue queue)
 {
-	__shared__ int stackStorage[kBvhShortStack * kThreads];
-	traceQueueClosest<kThreads>(bvh, queue, stackStorage);
+	__shared__ LeafSlots slots[kThreads / 32];
+	queueRewalk<kWide>(bvh, queue, slots);
+}
+
+template<bool kWide>
+__global__ void __launch_bounds__(128, 8) walkQueueKernel(BvhView bvh, RayQueue queue)
+{
+	__shared__ LeafSlots slots[4];
+	queueWalk<kWide>(bvh, queue, slots);
 }
 
 __global__ void __launch_bounds__(kGiThreads, RESTIR_GI_TEMPORAL_MIN_BLOCKS) giTemporalShadeKernel(const RestirParams P,
@@ -1112,11 +1121,6 @@ __global__ void __launch_bounds__(128, RESTIR_SPECULAR_MIN_BLOCKS) specularShade
 	specularFinish(g, r, hit, hitPosition, hitId, previousHdr, specularHistory, out, i);
 }
 
-__global__ void __launch_bounds__(128) traceQueueWalkKernel(BvhView bvh, RayQueue queue)
-{
-	traceQueueClosest<128, true>(bvh, queue, nullptr);
-}
-
 GiBindings bindings(const RestirGBuffer* gb, const RestirGiHistory* history, const uint32_t* grid, const float* shadowAtlas,
 	const uint16_t* surfaceLight)
 {
@@ -1238,7 +1242,7 @@ struct TemporalWorkspace
 	uint64_t bytes;
 };
 
-// [2 counters][rays 32 B x n][hit triangles 4 B x n][hit distances 4 B x n][screen hits 16 B x n]
+// [3 counters][rays 32 B x n][hit triangles 4 B x n][hit distances 4 B x n][screen hits 16 B x n]
 // [slots 4 B x n], each region starting on 256 bytes; n = GI pixels x initial candidates. With the
 // radiance cache: [queries 64 B x r][values 8 B x r], r = n + GI pixels, then the training batch of
 // s samples: [rays 32 B][hit triangles 4 B][hit distances 4 B][2 counters][training queries 64 B]
@@ -1255,7 +1259,7 @@ TemporalWorkspace layoutTemporalWorkspace(const RestirParams* p, void* base)
 		return start;
 	};
 	TemporalWorkspace w = {};
-	uint32_t* counters = reinterpret_cast<uint32_t*>(region(2 * sizeof(uint32_t)));
+	uint32_t* counters = reinterpret_cast<uint32_t*>(region(3 * sizeof(uint32_t)));
 	w.queue.count = counters;
 	w.queue.claimed = counters + 1;
 	w.queue.rays = reinterpret_cast<float4*>(region(n * 32));
@@ -1290,43 +1294,52 @@ TemporalWorkspace layoutTemporalWorkspace(const RestirParams* p, void* base)
 	return w;
 }
 
-// One resident grid of a queue tracer of 128 threads per block: SMs x blocks
-// that fit on one SM.
-int residentBlocks(const void* kernel)
+// One resident grid of a queue tracer: SMs x blocks that fit on one SM (or
+// blocksPerSm, when that is fewer), looked up once per kernel (not inside a
+// stream capture on later calls).
+template<typename Kernel>
+int residentBlocks(Kernel kernel, int threads, uint32_t blocksPerSm)
 {
-	int device = 0, sms = 148, perSm = 0;
+	int device = 0, sms = 148, fit = 0;
 	if (cudaGetDevice(&device) == cudaSuccess)
 	{
 		cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
 	}
-	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, kernel, 128, 0) != cudaSuccess || perSm < 1)
+	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, threads, 0) != cudaSuccess || fit < 1)
 	{
-		perSm = 1;
+		fit = 1;
 	}
-	return sms * perSm;
+	return sms * (blocksPerSm > 0u && int(blocksPerSm) < fit ? int(blocksPerSm) : fit);
 }
 
-int persistentBlocks()
+template<bool kWide, int kThreads>
+int launchNearest(const BvhView& bvh, const RayQueue& q, uint32_t blocksPerSm, cudaStream_t s)
 {
-	static int blocks = 0;
-	if (blocks == 0)
-	{
-		blocks = residentBlocks(reinterpret_cast<const void*>(traceQueueKernel));
-	}
-	return blocks;
+	static const int most = residentBlocks(traceQueueKernel<kWide, kThreads>, kThreads, 0u);
+	static const int mostRewalk = residentBlocks(rewalkQueueKernel<kWide, kThreads>, kThreads, 0u);
+	static const int sms = residentBlocks(traceQueueKernel<kWide, kThreads>, kThreads, 1u);
+	const int limit = blocksPerSm > 0u ? int(min(blocksPerSm, 32u)) * sms : most;
+	traceQueueKernel<kWide, kThreads><<<min(limit, most), kThreads, 0, s>>>(bvh, q);
+	rewalkQueueKernel<kWide, kThreads><<<mostRewalk, kThreads, 0, s>>>(bvh, q);
+	return launchStatus();
 }
 
-int walkBlocks()
+template<int kThreads = 128>
+int launchQueueTracer(const BvhView& bvh, const RayQueue& q, cudaStream_t s, uint32_t blocksPerSm = 0u)
 {
-	static int blocks = 0;
-	if (blocks == 0)
-	{
-		blocks = residentBlocks(reinterpret_cast<const void*>(traceQueueWalkKernel));
-	}
-	return blocks;
+	return wideRows(bvh) ? launchNearest<true, kThreads>(bvh, q, blocksPerSm, s)
+		: launchNearest<false, kThreads>(bvh, q, blocksPerSm, s);
 }
 
-// The specular wavefront's workspace: [2 counters][rays 32 B x n][hit triangles
+template<bool kWide>
+int launchWalk(const BvhView& bvh, const RayQueue& q, cudaStream_t s)
+{
+	static const int blocks = residentBlocks(walkQueueKernel<kWide>, 128, 0u);
+	walkQueueKernel<kWide><<<blocks, 128, 0, s>>>(bvh, q);
+	return launchStatus();
+}
+
+// The specular wavefront's workspace: [3 counters][rays 32 B x n][hit triangles
 // 4 B x n][hit distances 4 B x n][records 16 B x n], each region starting on 256
 // bytes; n = GI pixels.
 struct SpecularWorkspace
@@ -1348,7 +1361,7 @@ SpecularWorkspace layoutSpecularWorkspace(const RestirParams* p, void* base)
 		return start;
 	};
 	SpecularWorkspace w = {};
-	uint32_t* counters = reinterpret_cast<uint32_t*>(region(2 * sizeof(uint32_t)));
+	uint32_t* counters = reinterpret_cast<uint32_t*>(region(3 * sizeof(uint32_t)));
 	w.queue.count = counters;
 	w.queue.claimed = counters + 1;
 	w.queue.rays = reinterpret_cast<float4*>(region(n * 32));
@@ -1395,9 +1408,9 @@ extern "C" int restir_gi_temporal_wavefront(const RestirParams* params, const Re
 	cudaStream_t s = asStream(stream);
 	const int groups = int((params->gi_width + 3) / 4 * ((params->gi_height + 7) / 8));
 	const int blocks = (groups + kGiWarps - 1) / kGiWarps;
-	cudaMemsetAsync(workspace, 0, 2 * sizeof(uint32_t), s);
+	cudaMemsetAsync(workspace, 0, 3 * sizeof(uint32_t), s);
 	giCandidatesKernel<<<blocks, kGiThreads, 0, s>>>(*params, bvh, b, w.records, w.queue);
-	traceQueueKernel<<<persistentBlocks(), 128, 0, s>>>(bvh, w.queue);
+	launchQueueTracer(bvh, w.queue, s);
 	giTemporalShadeKernel<<<blocks, kGiThreads, 0, s>>>(*params, bvh, b, w.records, w.queue);
 	return launchStatus();
 }
@@ -1432,9 +1445,16 @@ extern "C" int restir_gi_specular_wavefront(const RestirParams* params, const Re
 	const BvhView bvh = makeBvhView(scene);
 	cudaStream_t s = asStream(stream);
 	dim3 grid((params->gi_width + 15) / 16, (params->gi_height + 7) / 8);
-	cudaMemsetAsync(workspace, 0, 2 * sizeof(uint32_t), s);
+	cudaMemsetAsync(workspace, 0, 3 * sizeof(uint32_t), s);
 	specularRaysKernel<<<grid, 128, 0, s>>>(*params, bvh, b, w.records, w.queue);
-	traceQueueWalkKernel<<<walkBlocks(), 128, 0, s>>>(bvh, w.queue);
+	if (wideRows(bvh))
+	{
+		launchWalk<true>(bvh, w.queue, s);
+	}
+	else
+	{
+		launchWalk<false>(bvh, w.queue, s);
+	}
 	specularShadeKernel<<<grid, 128, 0, s>>>(*params, bvh, b, w.records, w.queue, previous_hdr, specular_history, specular);
 	return launchStatus();
 }
@@ -1450,7 +1470,7 @@ namespace restir
 namespace
 {
 
-// [2 counters][rays 32 B x c][hit triangles 4 B x c][hit distances 4 B x c], each on 256 bytes.
+// [3 counters][rays 32 B x c][hit triangles 4 B x c][hit distances 4 B x c], each on 256 bytes.
 RayQueue layoutQueue(void* base, uint32_t capacity, uint64_t* bytes)
 {
 	char* at = static_cast<char*>(base);
@@ -1462,7 +1482,7 @@ RayQueue layoutQueue(void* base, uint32_t capacity, uint64_t* bytes)
 		return start;
 	};
 	RayQueue q;
-	uint32_t* counters = reinterpret_cast<uint32_t*>(region(2 * sizeof(uint32_t)));
+	uint32_t* counters = reinterpret_cast<uint32_t*>(region(3 * sizeof(uint32_t)));
 	q.count = counters;
 	q.claimed = counters + 1;
 	q.rays = reinterpret_cast<float4*>(region(uint64_t(capacity) * 32));
@@ -1496,34 +1516,6 @@ bool aligned(const void* p)
 	return p != nullptr && (reinterpret_cast<uintptr_t>(p) & 255u) == 0u;
 }
 
-template<int kThreads>
-int launchQueueTracer(const BvhView& bvh, const RayQueue& q, uint32_t blocksPerSm, cudaStream_t s)
-{
-	// SM count and resident blocks, queried once (not inside a stream capture on later calls).
-	static int sms = 0, fit = 0;
-	if (sms == 0)
-	{
-		int device = 0;
-		sms = 148;
-		if (cudaGetDevice(&device) == cudaSuccess)
-		{
-			cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-		}
-		if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, traceQueueSizedKernel<kThreads>, kThreads, 0) != cudaSuccess
-			|| fit < 1)
-		{
-			fit = 1;
-		}
-	}
-	int perSm = fit;
-	if (blocksPerSm > 0u && int(blocksPerSm) < perSm)
-	{
-		perSm = int(blocksPerSm);
-	}
-	traceQueueSizedKernel<kThreads><<<sms * perSm, kThreads, 0, s>>>(bvh, q);
-	return launchStatus();
-}
-
 } // namespace
 } // namespace restir
 
@@ -1540,7 +1532,7 @@ extern "C" int restir_ray_queue_reset(void* queue, void* stream)
 	{
 		return RESTIR_ERROR_INVALID_ARGUMENT;
 	}
-	return cudaMemsetAsync(queue, 0, 2 * sizeof(uint32_t), asStream(stream)) == cudaSuccess ? RESTIR_OK : RESTIR_ERROR_LAUNCH;
+	return cudaMemsetAsync(queue, 0, 3 * sizeof(uint32_t), asStream(stream)) == cudaSuccess ? RESTIR_OK : RESTIR_ERROR_LAUNCH;
 }
 
 extern "C" uint64_t restir_gi_candidate_records_bytes(const RestirParams* params)
@@ -1590,11 +1582,11 @@ extern "C" int restir_trace_queue(const RestirScene* scene, void* queue, uint32_
 	switch (threads)
 	{
 	case 64:
-		return launchQueueTracer<64>(bvh, q, blocks_per_sm, s);
+		return launchQueueTracer<64>(bvh, q, s, blocks_per_sm);
 	case 128:
-		return launchQueueTracer<128>(bvh, q, blocks_per_sm, s);
+		return launchQueueTracer<128>(bvh, q, s, blocks_per_sm);
 	case 256:
-		return launchQueueTracer<256>(bvh, q, blocks_per_sm, s);
+		return launchQueueTracer<256>(bvh, q, s, blocks_per_sm);
 	default:
 		return RESTIR_ERROR_INVALID_ARGUMENT;
 	}
@@ -1987,9 +1979,9 @@ extern "C" int restir_gi_temporal_cached(const RestirParams* params, const Resti
 	const int blocks = (groups + kGiWarps - 1) / kGiWarps;
 	const uint32_t candidates = w.queue.capacity;
 	const uint32_t pixels = params->gi_width * params->gi_height;
-	cudaMemsetAsync(workspace, 0, 2 * sizeof(uint32_t), s);
+	cudaMemsetAsync(workspace, 0, 3 * sizeof(uint32_t), s);
 	giCandidatesKernel<<<blocks, kGiThreads, 0, s>>>(*params, bvh, b, w.records, w.queue);
-	traceQueueKernel<<<persistentBlocks(), 128, 0, s>>>(bvh, w.queue);
+	launchQueueTracer(bvh, w.queue, s);
 	if (candidates > 0u)
 	{
 		candidateQueryKernel<<<gridFor(candidates), 128, 0, s>>>(*params, bvh, b, w.records, w.queue, w.cache.queries);
@@ -2123,13 +2115,13 @@ extern "C" int restir_cache_train_frame(const RestirParams* params, const Restir
 	// the frame's ray budget is the same as with visible-surface rows only.
 	const uint32_t first = (c.samples + 1u) / 2u;
 	const uint32_t second = c.samples - first;
-	cudaMemsetAsync(c.trainQueue.claimed, 0, sizeof(uint32_t), s);
+	cudaMemsetAsync(c.trainQueue.claimed, 0, 2 * sizeof(uint32_t), s);
 	if (second > 0u)
 	{
 		trainingSecondRaysKernel<<<gridFor(second), 128, 0, s>>>(*params, bvh, b, c, first, second);
 	}
 	trainingRaysKernel<<<gridFor(first), 128, 0, s>>>(*params, bvh, b, c, first);
-	traceQueueKernel<<<persistentBlocks(), 128, 0, s>>>(bvh, c.trainQueue);
+	launchQueueTracer(bvh, c.trainQueue, s);
 	trainingHitsKernel<<<gridFor(c.samples), 128, 0, s>>>(*params, bvh, b, c, 0u, c.samples);
 	int status = restir_cache_query(cache_config, cache_state, reinterpret_cast<const float*>(c.hitQueries), c.samples,
 		c.hitValues, stream);

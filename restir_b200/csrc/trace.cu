@@ -1,8 +1,9 @@
-// restir_trace: a fixed ray set through the BVH (bvh.sh:298-319), one thread
-// per ray. Closest-hit rays keep their short stack in shared memory,
-// interleaved so that the 32 lanes of a warp touch 32 different banks.
-// RESTIR_TRACE_CLOSEST_QUEUE runs the same closest-hit traversal through the
-// persistent queue tracer (wavefront.cuh): the ray set is the queue.
+// restir_trace: a fixed ray set through the BVH (bvh.sh:298-319). Each warp
+// takes a part of the set (warptrace.cuh), with a ray per lane or per group of
+// four lanes, or each thread one ray, by the size of the set and the scene; the
+// lock-step and the watertight walks run one thread per ray.
+// RESTIR_TRACE_CLOSEST_QUEUE always takes the parts, whose warps run the queue
+// tracer's loop. Nothing is allocated: a warp's part is its queue.
 #include "bvh.cuh"
 #include "wavefront.cuh"
 #include "watertight.cuh"
@@ -14,63 +15,172 @@ namespace
 
 constexpr int kTraceBlock = 128;
 
-__global__ void __launch_bounds__(kTraceBlock) traceKernel(BvhView bvh, const float4* __restrict__ rays,
-	int32_t* __restrict__ hitTriangle, float* __restrict__ hitDistance, uint32_t n, int kind)
+// Which kernel traces a ray set, by its size n and the scene's nodes. Measured
+// on random rays (us; one thread a ray / four lanes a ray / warp with leaves
+// tested together):
+//   any hit, 1M-triangle city, n 1,000: 81 / 47 / 87; 16,000: 105 / 75 / 129;
+//     64,000: 109 / 119 / 136; 400,000: 282 / 336 / 256;
+//   any hit, Cornell box, 16,000: 21 / 15 / 23; 400,000: 54 / 77 / 60;
+//   stackless, city, 16,000: 812 / 587 / 978; 1,000,000: - / 4,080 / 3,180;
+//   closest, city, 1,000: 378 / - / 320; 400,000: 1,247 / - / 1,018;
+//   closest, Cornell box, 1,000: 19 / - / 25; 400,000: 64 / - / 83.
+// So up to a group of four lanes for each ray that the SMs hold at once (148 x
+// 32 warps x 8), walks are latency-bound and take four lanes; until every lane
+// has two rays, one thread each is enough; past that, and for nearest hits,
+// the warp's shared leaves win, unless the scene is so small that a ray visits
+// some twenty nodes and half of the time goes to fetching the longer code.
+constexpr uint32_t kFourLaneRays = 148u * 32u * 8u;
+constexpr uint32_t kThreadRays = 148u * 32u * 32u * 2u;
+constexpr int kSmallScene = 4096;
+
+
+// A contiguous part of the ray set, one per warp: its lanes take the part's
+// rays as theirs end, without an atomic.
+template<int kKind, int kLanes>
+struct PartSource
 {
-	__shared__ int stack[kBvhShortStack * kTraceBlock];
+	static constexpr int kCount = kKind;
+	RayArrays arrays;
+	uint32_t next, end;
+
+	__device__ __forceinline__ void take(bool idle, bool& more, Ray& r)
+	{
+		const unsigned mask = idleMask<kLanes>(idle);
+		const uint32_t wanted = uint32_t(__popc(mask));
+		const uint32_t left = end - next;
+		const uint32_t rank = uint32_t(idleRank<kLanes>(mask));
+		if (idle && rank < left)
+		{
+			arrays.load(int(next + rank), r);
+		}
+		next += min(wanted, left);
+		more = left > wanted;
+	}
+	__device__ __forceinline__ void store(const Ray& r) const { arrays.store(r); }
+};
+
+__device__ __forceinline__ bool warpPart(uint32_t n, uint32_t part, uint32_t& first, uint32_t& end)
+{
+	const uint64_t at = (uint64_t(blockIdx.x) * (kTraceBlock / 32) + (threadIdx.x >> 5)) * part;
+	first = uint32_t(at);
+	end = uint32_t(min(at + part, uint64_t(n)));
+	return at < n;
+}
+
+template<bool kWide>
+__global__ void __launch_bounds__(kTraceBlock, 8) nearestPartsKernel(BvhView bvh, RayArrays arrays, uint32_t n, uint32_t part)
+{
+	__shared__ NearestStorage storage[kTraceBlock / 32];
+	uint32_t first, end;
+	if (!warpPart(n, part, first, end))
+	{
+		return; // whole warp
+	}
+	PartSource<RESTIR_COUNT_CLOSEST, 1> source{ arrays, first, end };
+	traceNearest<kWide>(bvh, source, storage[threadIdx.x >> 5]);
+	__syncwarp(); // the warp's stores
+	MarkedSource<4> marked{ arrays, first, end, nullptr };
+	traceWalks<false, kWide, 4>(bvh, marked, storage[threadIdx.x >> 5].leaves);
+}
+
+template<bool kAny, bool kWide, int kLanes>
+__global__ void __launch_bounds__(kTraceBlock, 8) walkPartsKernel(BvhView bvh, RayArrays arrays, uint32_t n, uint32_t part)
+{
+	__shared__ LeafSlots slots[kTraceBlock / 32];
+	uint32_t first, end;
+	if (!warpPart(n, part, first, end))
+	{
+		return; // whole warp
+	}
+	PartSource<RESTIR_COUNT_ANY, kLanes> source{ arrays, first, end };
+	traceWalks<kAny, kWide, kLanes>(bvh, source, slots[threadIdx.x >> 5]);
+}
+
+// One thread per ray, a kernel per kind (each fetches its own kind's code only:
+// 1,000 any-hit rays in the Cornell box take 21 us against 23 us in one kernel
+// for all kinds).
+template<int kKind>
+__global__ void __launch_bounds__(kTraceBlock) traceKernel(BvhView bvh, RayArrays arrays, uint32_t n)
+{
+	__shared__ int stack[kKind == RESTIR_TRACE_CLOSEST ? kBvhShortStack * kTraceBlock : 1];
 	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
 	if (i >= n)
 	{
 		return;
 	}
-	float4 a = __ldg(rays + 2 * i);
-	float4 b = __ldg(rays + 2 * i + 1);
-	V3 o = v3(a.x, a.y, a.z);
-	V3 d = v3(b.x, b.y, b.z);
-	float distance = a.w;
-	int hit = -1;
-	if (kind == RESTIR_TRACE_CLOSEST)
+	Ray r;
+	arrays.load(int(i), r);
+	const float length = r.distance;
+	if (kKind == RESTIR_TRACE_CLOSEST)
 	{
-		hit = traceBvh(bvh, o, d, a.w, false, distance, stack + threadIdx.x, kTraceBlock);
+		r.hit = traceBvh(bvh, r.o, r.d, length, false, r.distance, stack + threadIdx.x, kTraceBlock);
 	}
-	else if (kind == RESTIR_TRACE_ANY)
+	else if (kKind == RESTIR_TRACE_ANY || kKind == RESTIR_TRACE_CLOSEST_STACKLESS)
 	{
-		hit = traceBvh(bvh, o, d, a.w, true, distance, nullptr, 0);
+		r.hit = traceBvh(bvh, r.o, r.d, length, kKind == RESTIR_TRACE_ANY, r.distance, nullptr, 0);
 	}
-	else if (kind == RESTIR_TRACE_CLOSEST_STACKLESS)
+	else if (kKind == RESTIR_TRACE_ANY_WAVE)
 	{
-		hit = traceBvh(bvh, o, d, a.w, false, distance, nullptr, 0);
-	}
-	else if (kind == RESTIR_TRACE_ANY_WAVE)
-	{
-		hit = traceVisibility(bvh, o, d, a.w, distance, true);
+		r.hit = traceVisibility(bvh, r.o, r.d, length, r.distance, true);
 	}
 	else
 	{
-		hit = traceWatertight(bvh, o, d, distance);
+		r.hit = traceWatertight(bvh, r.o, r.d, r.distance);
 	}
-	hitTriangle[i] = hit;
-	hitDistance[i] = distance;
+	arrays.store(r);
 }
 
-__global__ void __launch_bounds__(kTraceBlock) traceQueueKernel(BvhView bvh, RayQueue queue)
+template<int kKind>
+void launchThreads(const BvhView& bvh, const RayArrays& arrays, uint32_t n, cudaStream_t s)
 {
-	__shared__ int stack[kBvhShortStack * kTraceBlock];
-	traceQueueClosest<kTraceBlock>(bvh, queue, stack);
+	traceKernel<kKind><<<(n + kTraceBlock - 1) / kTraceBlock, kTraceBlock, 0, s>>>(bvh, arrays, n);
 }
 
-int residentQueueBlocks()
+// Rays per warp: as few as fill the SMs once (148 x 32 warps resident), a
+// multiple of the lanes' or groups' number, then four times that, so that
+// lanes whose rays end early have more to take.
+uint32_t partOf(uint32_t n, uint32_t takers)
 {
-	int device = 0, sms = 148, perSm = 0;
-	if (cudaGetDevice(&device) == cudaSuccess)
+	return n > 148u * 32u * takers ? 4u * takers : takers;
+}
+
+uint32_t partBlocks(uint32_t n, uint32_t part)
+{
+	const uint64_t warps = (uint64_t(n) + part - 1u) / part;
+	return uint32_t((warps + kTraceBlock / 32 - 1) / (kTraceBlock / 32));
+}
+
+template<bool kAny, bool kWide>
+void launchWalks(const BvhView& bvh, const RayArrays& arrays, uint32_t n, cudaStream_t s)
+{
+	if (n <= kFourLaneRays)
 	{
-		cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+		const uint32_t part = partOf(n, 8u);
+		walkPartsKernel<kAny, kWide, 4><<<partBlocks(n, part), kTraceBlock, 0, s>>>(bvh, arrays, n, part);
 	}
-	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, traceQueueKernel, kTraceBlock, 0) != cudaSuccess || perSm < 1)
+	else
 	{
-		perSm = 1;
+		const uint32_t part = partOf(n, 32u);
+		walkPartsKernel<kAny, kWide, 1><<<partBlocks(n, part), kTraceBlock, 0, s>>>(bvh, arrays, n, part);
 	}
-	return sms * perSm;
+}
+
+template<bool kWide>
+void launchParts(const BvhView& bvh, const RayArrays& arrays, uint32_t n, int kind, cudaStream_t s)
+{
+	if (kind == RESTIR_TRACE_CLOSEST || kind == RESTIR_TRACE_CLOSEST_QUEUE)
+	{
+		const uint32_t part = partOf(n, 32u);
+		nearestPartsKernel<kWide><<<partBlocks(n, part), kTraceBlock, 0, s>>>(bvh, arrays, n, part);
+	}
+	else if (kind == RESTIR_TRACE_ANY)
+	{
+		launchWalks<true, kWide>(bvh, arrays, n, s);
+	}
+	else
+	{
+		launchWalks<false, kWide>(bvh, arrays, n, s);
+	}
 }
 
 } // namespace
@@ -93,31 +203,36 @@ extern "C" int restir_trace(const RestirParams* params, const RestirScene* scene
 	}
 	BvhView bvh = makeBvhView(scene);
 	cudaStream_t s = asStream(stream);
-	if (kind == RESTIR_TRACE_CLOSEST_QUEUE)
+	const RayArrays arrays = { reinterpret_cast<const float4*>(rays), hit_triangle, hit_distance };
+	const bool small = bvh.nodeCount <= kSmallScene;
+	const bool threads = n > kFourLaneRays && (small || n <= kThreadRays);
+	if (kind == RESTIR_TRACE_ANY_WAVE)
 	{
-		// The claim counter lives in stream-ordered memory, so that calls on
-		// different streams do not share it.
-		uint32_t* claimed = nullptr;
-		if (cudaMallocAsync(reinterpret_cast<void**>(&claimed), sizeof(uint32_t), s) != cudaSuccess)
-		{
-			cudaGetLastError();
-			return RESTIR_ERROR_OUT_OF_MEMORY;
-		}
-		cudaMemsetAsync(claimed, 0, sizeof(uint32_t), s);
-		RayQueue q;
-		q.rays = const_cast<float4*>(reinterpret_cast<const float4*>(rays));
-		q.hitTriangle = hit_triangle;
-		q.hitDistance = hit_distance;
-		q.count = nullptr;
-		q.claimed = claimed;
-		q.capacity = n;
-		static const int blocks = residentQueueBlocks();
-		traceQueueKernel<<<blocks, kTraceBlock, 0, s>>>(bvh, q);
-		const int status = launchStatus();
-		cudaFreeAsync(claimed, s);
-		return status;
+		launchThreads<RESTIR_TRACE_ANY_WAVE>(bvh, arrays, n, s);
 	}
-	traceKernel<<<(n + kTraceBlock - 1) / kTraceBlock, kTraceBlock, 0, s>>>(
-		bvh, reinterpret_cast<const float4*>(rays), hit_triangle, hit_distance, n, kind);
+	else if (kind == RESTIR_TRACE_CLOSEST_WATERTIGHT)
+	{
+		launchThreads<RESTIR_TRACE_CLOSEST_WATERTIGHT>(bvh, arrays, n, s);
+	}
+	else if (kind == RESTIR_TRACE_CLOSEST && small)
+	{
+		launchThreads<RESTIR_TRACE_CLOSEST>(bvh, arrays, n, s);
+	}
+	else if (kind == RESTIR_TRACE_ANY && threads)
+	{
+		launchThreads<RESTIR_TRACE_ANY>(bvh, arrays, n, s);
+	}
+	else if (kind == RESTIR_TRACE_CLOSEST_STACKLESS && threads)
+	{
+		launchThreads<RESTIR_TRACE_CLOSEST_STACKLESS>(bvh, arrays, n, s);
+	}
+	else if (wideRows(bvh))
+	{
+		launchParts<true>(bvh, arrays, n, kind, s);
+	}
+	else
+	{
+		launchParts<false>(bvh, arrays, n, kind, s);
+	}
 	return launchStatus();
 }

@@ -3,21 +3,13 @@
 //
 // A producer pass appends rays to a queue in global memory (a warp's lanes
 // take consecutive slots: one __ballot_sync, one atomicAdd per warp). The
-// tracer below runs one resident grid; each lane holds one ray and advances
-// it one node per loop iteration, and as soon as its ray finishes it takes
-// the next unclaimed ray (again one atomicAdd per warp for all lanes that
-// need one). Lanes therefore stay in the same traversal loop instead of
-// idling behind the longest ray of their warp.
-//
-// The per-ray algorithm is the reference's nearest-first short-stack
-// traversal (bvh.sh:216-295) written as a resumable state machine: the same
-// nodes in the same order, the same step cap, the same stackless fallback,
-// so hit ids and distances are identical to traceShortStack's. The tracer's
-// walk form runs the stackless walk (bvh.sh:140-174) the same way, for the
-// rays of the fragment-shader passes.
+// tracer below runs one resident grid; each lane holds one ray (warptrace.cuh),
+// and lanes whose rays have ended take the next unclaimed ones. Lanes therefore
+// stay in the same traversal loop instead of idling behind the longest ray of
+// their warp.
 #pragma once
 
-#include "bvh.cuh"
+#include "warptrace.cuh"
 
 namespace restir
 {
@@ -30,7 +22,7 @@ struct RayQueue
 	int* hitTriangle;
 	float* hitDistance;
 	uint32_t* count;    // rays appended by the producer; null: capacity rays
-	uint32_t* claimed;  // rays taken by the tracer
+	uint32_t* claimed;  // rays taken by the tracer; next to it, rays looked through by the re-walk
 	uint32_t capacity;
 };
 
@@ -62,279 +54,146 @@ __device__ __forceinline__ int queuePush(const RayQueue& q, bool push, V3 origin
 	return int(slot);
 }
 
-// One lane's traversal state (registers), its short stack in shared memory.
-struct ShortStackState
+__device__ __forceinline__ uint32_t queuedRays(const RayQueue& q)
 {
-	V3 o, d, inv;
-	float distance;
-	int hit;          // nearest hit of the short-stack walk
-	int fallbackHit;  // nearest hit of the stackless re-walk
-	int node;
-	int stackTop;
-	int stackCount;
-	int step;
-	bool dropped;
-	int phase;        // 0 short stack, 1 stackless re-walk, 2 done
-	TraceWork work;
+	return q.count != nullptr ? min(*q.count, q.capacity) : q.capacity;
+}
+
+// Rays and hits in restir_trace's layout.
+struct RayArrays
+{
+	const float4* rays;
+	int* hitTriangle;
+	float* hitDistance;
+
+	__device__ __forceinline__ void load(int i, Ray& r) const
+	{
+		const float4 a = rays[2 * size_t(i)];
+		const float4 c = rays[2 * size_t(i) + 1];
+		r.o = v3(a.x, a.y, a.z);
+		r.d = v3(c.x, c.y, c.z);
+		r.distance = a.w;
+		r.hit = -1;
+		r.index = i;
+	}
+	__device__ __forceinline__ void store(const Ray& r) const
+	{
+		hitTriangle[r.index] = r.hit;
+		hitDistance[r.index] = r.distance;
+	}
 };
 
-__device__ __forceinline__ void startShortStack(ShortStackState& s, const BvhView& b, V3 o, V3 d, float tmax)
+// A queue as a source: one atomicAdd per warp claims rays for all takers.
+template<int kKind, int kLanes>
+struct QueueSource
 {
-	s.o = o;
-	s.d = d;
-	s.inv = bvhInverseDirection(d);
-	s.distance = tmax;
-	s.hit = -1;
-	s.fallbackHit = -1;
-	s.node = 0;
-	s.stackTop = 0;
-	s.stackCount = 0;
-	s.step = 0;
-	s.dropped = false;
-	s.work = TraceWork();
-	s.phase = 0;
-	++s.work.nodes;
-	if (!b.available() || intersectBox(o, s.inv, b.row(0).xyz(), b.row(1).xyz(), s.distance) < 0.0f)
-	{
-		s.phase = 2;
-	}
-}
+	static constexpr int kCount = kKind;
+	const RayQueue& q;
+	RayArrays arrays;
+	uint32_t total;
 
-// A ray of the stackless walk alone (the fragment-shader passes): phase 1
-// from the root, whose box the walk tests in its first step.
-__device__ __forceinline__ void startStacklessWalk(ShortStackState& s, V3 o, V3 d, float tmax)
-{
-	s.o = o;
-	s.d = d;
-	s.inv = bvhInverseDirection(d);
-	s.distance = tmax;
-	s.hit = -1;
-	s.fallbackHit = -1;
-	s.node = 0;
-	s.stackTop = 0;
-	s.stackCount = 0;
-	s.step = 0;
-	s.dropped = false;
-	s.work = TraceWork();
-	s.phase = 1;
-}
+	__device__ __forceinline__ explicit QueueSource(const RayQueue& queue)
+		: q(queue), arrays{ queue.rays, queue.hitTriangle, queue.hitDistance }, total(queuedRays(queue))
+	{
+	}
+	__device__ __forceinline__ void take(bool idle, bool& more, Ray& r) const
+	{
+		const unsigned mask = idleMask<kLanes>(idle);
+		const uint32_t wanted = uint32_t(__popc(mask));
+		uint32_t start = 0;
+		if ((threadIdx.x & 31u) == 0u)
+		{
+			start = atomicAdd(q.claimed, wanted);
+		}
+		start = __shfl_sync(0xffffffffu, start, 0);
+		more = start < total && total - start > wanted;
+		const uint32_t mine = start + uint32_t(idleRank<kLanes>(mask));
+		if (idle && mine >= start && mine < total)
+		{
+			arrays.load(int(mine), r);
+		}
+	}
+	__device__ __forceinline__ void store(const Ray& r) const { arrays.store(r); }
+};
 
-// The end of the short-stack walk: the stackless re-walk if entries were dropped.
-__device__ __forceinline__ void endShortStack(ShortStackState& s)
+// The marked rays (markedHit) among the first `end` of a ray set: a source for
+// traceWalks. The warp looks through 32 consecutive rays at a time, the next
+// ones no warp has claimed (claimed), or the next of its own part (null).
+template<int kLanes>
+struct MarkedSource
 {
-	if (s.step == kBvhMaxSteps)
-	{
-		reportTruncatedRay();
-	}
-	if (s.dropped)
-	{
-		s.phase = 1;
-		s.node = 0;
-		s.step = 0;
-	}
-	else
-	{
-		s.phase = 2;
-	}
-}
+	static constexpr int kCount = -1;
+	RayArrays arrays;
+	uint32_t next, end;
+	uint32_t* claimed;
+	uint32_t base = 0u;
+	unsigned pending = 0u; // marked rays from base on
 
-// traceStacklessWalk (bvh.sh:140-174), one node per call (the short stack's
-// re-walk, phase 1) or, with kPair, one or two (a whole ray started by
-// startStacklessWalk): the rows of the node after this one are fetched with
-// this node's, and when the walk goes on to it (a box passed, or a leaf) it
-// is visited in the same call, so that fetch's latency overlaps this node's
-// test. Nodes, order and step count are the walk's.
-template<bool kPair>
-__device__ __forceinline__ void stepStacklessWalk(ShortStackState& s, const BvhView& b)
-{
-	if (s.step >= kBvhMaxSteps || s.node >= b.nodeCount)
+	__device__ __forceinline__ void take(bool idle, bool& more, Ray& r)
 	{
-		if (s.step >= kBvhMaxSteps)
+		const unsigned lane = threadIdx.x & 31u;
+		unsigned mask = idleMask<kLanes>(idle);
+		while (mask != 0u)
 		{
-			reportTruncatedRay();
-		}
-		if (s.fallbackHit >= 0)
-		{
-			s.hit = s.fallbackHit;
-		}
-		s.phase = 2;
-		return;
-	}
-	const int following = s.node + 1;
-	const bool fetched = kPair && following < b.nodeCount;
-	const V4 node0 = b.row(s.node * 2);
-	const V4 node1 = b.row(s.node * 2 + 1);
-	V4 next0 = node0, next1 = node1;
-	if (fetched)
-	{
-		next0 = b.row(following * 2);
-		next1 = b.row(following * 2 + 1);
-	}
-	auto visit = [&](const V4& row0, const V4& row1)
-	{
-		++s.work.nodes;
-		++s.step;
-		const bool leaf = row1.w >= 0.0f;
-		if (intersectBox(s.o, s.inv, row0.xyz(), row1.xyz(), s.distance) < 0.0f)
-		{
-			s.node = leaf ? s.node + 1 : int(-row1.w) - 1;
-			return;
-		}
-		if (leaf)
-		{
-			s.fallbackHit = intersectLeaf(b, s.o, s.d, int(row0.w), int(row1.w), s.distance, s.fallbackHit, s.work);
-		}
-		s.node = s.node + 1;
-	};
-	visit(node0, node1);
-	if (fetched && s.node == following && s.step < kBvhMaxSteps)
-	{
-		visit(next0, next1);
-	}
-}
-
-// Advances the traversal by one node.
-__device__ __forceinline__ void stepShortStack(ShortStackState& s, const BvhView& b, int* stack, int stride)
-{
-	if (s.phase == 0)
-	{
-		if (s.step >= kBvhMaxSteps)
-		{
-			endShortStack(s);
-			return;
-		}
-		V4 node0 = b.row(s.node * 2);
-		V4 node1 = b.row(s.node * 2 + 1);
-		if (node1.w >= 0.0f)
-		{
-			s.hit = intersectLeaf(b, s.o, s.d, int(node0.w), int(node1.w), s.distance, s.hit, s.work);
-		}
-		else
-		{
-			int left = s.node + 1;
-			int right = int(node0.w);
-			s.work.nodes += 2u;
-			float leftDistance = intersectBox(s.o, s.inv, b.row(left * 2).xyz(), b.row(left * 2 + 1).xyz(), s.distance);
-			float rightDistance = intersectBox(s.o, s.inv, b.row(right * 2).xyz(), b.row(right * 2 + 1).xyz(), s.distance);
-			bool visitLeft = leftDistance >= 0.0f;
-			bool visitRight = rightDistance >= 0.0f;
-			if (visitLeft && visitRight)
+			if (pending == 0u)
 			{
-				bool leftFirst = leftDistance <= rightDistance;
-				stack[(s.stackTop & (kBvhShortStack - 1)) * stride] = leftFirst ? right : left;
-				++s.stackTop;
-				if (s.stackCount == kBvhShortStack)
+				base = next;
+				if (claimed != nullptr)
 				{
-					s.dropped = true;
-				}
-				else
-				{
-					++s.stackCount;
-				}
-				s.node = leftFirst ? left : right;
-				++s.step;
-				return;
-			}
-			if (visitLeft || visitRight)
-			{
-				s.node = visitLeft ? left : right;
-				++s.step;
-				return;
-			}
-		}
-		if (s.stackCount == 0)
-		{
-			endShortStack(s);
-			return;
-		}
-		--s.stackTop;
-		--s.stackCount;
-		s.node = stack[(s.stackTop & (kBvhShortStack - 1)) * stride];
-		++s.step;
-		return;
-	}
-	if (s.phase == 1)
-	{
-		stepStacklessWalk<false>(s, b);
-	}
-}
-
-// The persistent closest-hit tracer over a queue. Launch with a whole number
-// of warps per block; stack: kBvhShortStack ints per thread of the block.
-// kWalk: every ray takes the stackless walk instead (traceBvh without a
-// stack, the fragment-shader passes; no stack storage).
-template<int kThreads, bool kWalk = false>
-__device__ inline void traceQueueClosest(const BvhView& b, const RayQueue& q, int* stackStorage)
-{
-	const unsigned lane = threadIdx.x & 31u;
-	int* stack = kWalk ? nullptr : stackStorage + threadIdx.x;
-	const uint32_t total = q.count != nullptr ? min(*q.count, q.capacity) : q.capacity;
-	ShortStackState s;
-	s.phase = 2;
-	int ray = -1;
-	bool exhausted = false;
-	for (;;)
-	{
-		// Lanes without a ray take the next ones, one atomic per warp.
-		const bool need = ray < 0 && !exhausted;
-		const unsigned needMask = __ballot_sync(0xffffffffu, need);
-		if (needMask != 0u)
-		{
-			uint32_t base = 0;
-			if (lane == uint32_t(__ffs(needMask) - 1))
-			{
-				base = atomicAdd(q.claimed, uint32_t(__popc(needMask)));
-			}
-			base = __shfl_sync(0xffffffffu, base, __ffs(needMask) - 1);
-			if (need)
-			{
-				const uint32_t index = base + uint32_t(__popc(needMask & ((1u << lane) - 1u)));
-				if (index < total)
-				{
-					ray = int(index);
-					float4 a = q.rays[2 * index];
-					float4 c = q.rays[2 * index + 1];
-					if (kWalk)
+					if (lane == 0u)
 					{
-						startStacklessWalk(s, v3(a.x, a.y, a.z), v3(c.x, c.y, c.z), a.w);
+						base = atomicAdd(claimed, 32u);
 					}
-					else
-					{
-						startShortStack(s, b, v3(a.x, a.y, a.z), v3(c.x, c.y, c.z), a.w);
-					}
+					base = __shfl_sync(0xffffffffu, base, 0);
 				}
-				else
+				if (base >= end)
 				{
-					exhausted = true;
+					more = false;
+					break;
 				}
+				next = base + 32u;
+				const uint32_t i = base + lane;
+				pending = __ballot_sync(0xffffffffu, i >= base && i < end && arrays.hitTriangle[i] < -1);
+				continue;
 			}
-		}
-		if (!__any_sync(0xffffffffu, ray >= 0))
-		{
-			break;
-		}
-		if (ray >= 0)
-		{
-			if (s.phase != 2)
+			// The first idle group takes the first marked ray.
+			if ((lane & ~unsigned(kLanes - 1)) == unsigned(__ffs(mask) - 1))
 			{
-				if (kWalk)
-				{
-					stepStacklessWalk<true>(s, b);
-				}
-				else
-				{
-					stepShortStack(s, b, stack, kThreads);
-				}
+				const int i = int(base) + __ffs(pending) - 1;
+				arrays.load(i, r);
+				r.hit = markedHit(arrays.hitTriangle[i]);
+				r.distance = arrays.hitDistance[i];
 			}
-			if (s.phase == 2)
-			{
-				q.hitTriangle[ray] = s.hit;
-				q.hitDistance[ray] = s.distance;
-				countWork(kWalk ? RESTIR_COUNT_ANY : RESTIR_COUNT_CLOSEST, s.work.nodes, s.work.triangles);
-				ray = -1;
-			}
+			mask &= mask - 1u;
+			pending &= pending - 1u;
 		}
 	}
+	__device__ __forceinline__ void store(const Ray& r) const { arrays.store(r); }
+};
+
+// The persistent tracers over a queue, for grids of whole warps. Nearest hits
+// take two launches: queueNearest marks the rays whose short stack dropped
+// entries, queueRewalk finishes those. queueWalk traces nearest hits by the
+// stackless walk alone (the fragment-shader passes).
+template<bool kWide>
+__device__ __forceinline__ void queueNearest(const BvhView& b, const RayQueue& q, NearestStorage* storage)
+{
+	QueueSource<RESTIR_COUNT_CLOSEST, 1> source(q);
+	traceNearest<kWide>(b, source, storage[threadIdx.x >> 5]);
+}
+
+template<bool kWide>
+__device__ __forceinline__ void queueRewalk(const BvhView& b, const RayQueue& q, LeafSlots* slots)
+{
+	MarkedSource<4> source{ { q.rays, q.hitTriangle, q.hitDistance }, 0u, queuedRays(q), q.claimed + 1 };
+	traceWalks<false, kWide, 4>(b, source, slots[threadIdx.x >> 5]);
+}
+
+template<bool kWide>
+__device__ __forceinline__ void queueWalk(const BvhView& b, const RayQueue& q, LeafSlots* slots)
+{
+	QueueSource<RESTIR_COUNT_ANY, 4> source(q);
+	traceWalks<false, kWide, 4>(b, source, slots[threadIdx.x >> 5]);
 }
 
 } // namespace restir

@@ -1,0 +1,95 @@
+"""The warp-cooperative traversal (csrc/warptrace.cuh) on scenes and ray counts
+at its edges: trees deep enough to drop short-stack entries, leaves of more than
+four triangles, partial warps and groups, each launch rule's limits, and a BVH
+buffer that starts on 16 bytes only. Hits and distances bit-exact vs the oracle.
+"""
+import numpy as np
+import pytest
+
+import oracle.binding as ob
+import restir_b200 as rb
+from tests.helpers import SceneSetup, make_scene, seeded_rays
+
+KINDS = [rb.TRACE_CLOSEST, rb.TRACE_ANY, rb.TRACE_CLOSEST_STACKLESS, rb.TRACE_CLOSEST_QUEUE]
+
+
+def large_leaves(setup: SceneSetup) -> SceneSetup:
+    """setup with a tree of this test's own over its triangles: leaves of 5 to 12 of them, sorted by x."""
+    data = setup.bvh.data.reshape(-1, 4)
+    n, offset = setup.bvh.desc.triangle_count, setup.bvh.desc.triangle_offset
+    triangles = data[offset:].reshape(n, 4, 4)
+    triangles = triangles[np.argsort(triangles[:, :3, 0].mean(1), kind="stable")]
+    bounds = np.concatenate([[0], np.cumsum(np.tile([5, 12, 9, 7, 8], n // 41 + 1))])
+    bounds = np.append(bounds[bounds < n], n)
+    nodes = []
+
+    def build(lo, hi):
+        corners = triangles[bounds[lo]:bounds[hi], :3, :3].reshape(-1, 3)
+        index = len(nodes)
+        nodes.append(None)
+        if hi - lo == 1:
+            a, b = bounds[lo], bounds[hi] - bounds[lo]
+        else:
+            build(lo, (lo + hi) // 2)
+            a = len(nodes)
+            build((lo + hi) // 2, hi)
+            b = -len(nodes) - 1
+        nodes[index] = [[*corners.min(0), a], [*corners.max(0), b]]
+
+    build(0, len(bounds) - 1)
+    rows = np.concatenate([np.array(nodes, np.float32).reshape(-1, 4), triangles.reshape(-1, 4)]).astype(np.float32)
+    setup.bvh_data, setup.node_count, setup.triangle_offset = rows.reshape(-1), len(nodes), 2 * len(nodes)
+    return setup
+
+
+def check(setup, rays, kind, offset=0):
+    import torch
+    n = len(rays)
+    ids, t = np.zeros(n, np.int32), np.zeros(n, np.float32)
+    ob.load().oracle_trace(None, setup.host_scene(), rays.ctypes.data, ids.ctypes.data, t.ctypes.data, n, kind)
+    scene = setup.device_scene()
+    data = setup.bvh_data if setup.bvh_data is not None else setup.bvh.data
+    rows = torch.zeros(data.size + 8, dtype=torch.float32, device="cuda")
+    rows[offset:offset + data.size] = torch.from_numpy(data).cuda()
+    scene.bvh = rows[offset:].data_ptr()
+    d_rays = torch.from_numpy(rays).cuda()
+    d_ids, d_t = torch.empty(n, dtype=torch.int32, device="cuda"), torch.empty(n, dtype=torch.float32, device="cuda")
+    rb.check(rb.load().restir_trace(None, scene, d_rays.data_ptr(), d_ids.data_ptr(), d_t.data_ptr(), n, kind, None),
+             "restir_trace")
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(d_ids.cpu().numpy(), ids)
+    np.testing.assert_array_equal(d_t.cpu().numpy().view(np.uint32), t.view(np.uint32))
+    rb.status_flags()  # some of these rays reach the step cap, as the oracle's do
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("n", [1, 31, 33, 1000, 37_888, 37_889, 303_105])
+def test_ray_counts(kind, n):
+    setup = make_scene(rb.SCENE_CITY, 0, 60_000)
+    check(setup, seeded_rays(setup, 303_105, seed=5)[::-1][:n].copy(), kind)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("triangles", [300, 4_000, 120_000])
+def test_scene_sizes(kind, triangles):
+    setup = make_scene(rb.SCENE_COURTYARD, 1, triangles)
+    check(setup, seeded_rays(setup, 50_000, seed=6), kind)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("n", [500, 310_000])
+def test_large_leaves(kind, n):
+    setup = large_leaves(make_scene(rb.SCENE_COURTYARD, 2, 20_000))
+    assert setup.node_count > 4096
+    check(setup, seeded_rays(setup, n, seed=7), kind)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS)
+def test_unaligned_rows(kind):
+    """16 bytes past a 32-byte boundary: the nodes are read with 128-bit loads."""
+    setup = make_scene(rb.SCENE_CITY, 0, 60_000)
+    check(setup, seeded_rays(setup, 20_000, seed=8), kind, offset=4)
