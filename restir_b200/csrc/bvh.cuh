@@ -115,6 +115,7 @@ __device__ __forceinline__ int intersectLeaf(const BvhView& b, V3 o, V3 d, int f
 	TraceWork& work)
 {
 	work.triangles += uint32_t(count);
+#pragma unroll 1
 	for (int t = first; t < first + count; ++t)
 	{
 		float h = intersectTriangle(o, d, b.vertex(t, 0), b.vertex(t, 1), b.vertex(t, 2));

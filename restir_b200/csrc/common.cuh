@@ -193,15 +193,22 @@ __device__ __forceinline__ void storeH4(uint16_t* p, int i, V4 v)
 	reinterpret_cast<uint2*>(p)[i] = q;
 }
 
+// u / 255 rounded once, for u = 0 .. 255: 1/255 as the sum of two floats, the
+// second's product added in one rounding, equals the division for all 256
+// (tests/test_numeric.py). Two instructions for the division's eleven; the GI
+// kernels decode a normal at every step of a depth-buffer march and fetch
+// their code from beyond the instruction cache.
+__device__ __forceinline__ float unorm8(uint32_t u)
+{
+	const float x = float(u);
+	return __fmaf_rn(x, 0x1.010102p-8f, x * -0x1.fdfdfep-33f);
+}
+
 // BGRA8 bytes, read back as (r, g, b, a).
 __device__ __forceinline__ V4 loadU8(const uint8_t* p, int i)
 {
 	uint32_t q = __ldg(reinterpret_cast<const uint32_t*>(p) + i);
-	return {
-		  float((q >> 16) & 0xffu) / 255.0f
-		, float((q >> 8) & 0xffu) / 255.0f
-		, float(q & 0xffu) / 255.0f
-		, float(q >> 24) / 255.0f };
+	return { unorm8((q >> 16) & 0xffu), unorm8((q >> 8) & 0xffu), unorm8(q & 0xffu), unorm8(q >> 24) };
 }
 
 __device__ __forceinline__ void storeU8(uint8_t* p, int i, V4 v)

@@ -109,3 +109,13 @@ def test_device_numeric_bit_identical():
         torch.cuda.synchronize()
         host = host_eval(4 if fn == 3 else fn, x)
         np.testing.assert_array_equal(d_out.cpu().numpy().view(np.uint32), host.view(np.uint32), err_msg=f"fn {fn}")
+
+
+def test_unorm8_two_term_product():
+    """The kernels' u / 255 (csrc/common.cuh unorm8): u * 1/255's head plus the rounded product with its tail, in one
+    rounding, equals the correctly rounded quotient for every byte."""
+    head, tail = np.float32(float.fromhex("0x1.010102p-8")), np.float32(float.fromhex("-0x1.fdfdfep-33"))
+    u = np.arange(256, dtype=np.float32)
+    # u * head (at most 32 bits) plus the small term is exact in binary64: rounding it to float is the fused operation.
+    fused = (u.astype(np.float64) * np.float64(head) + np.float64(u * tail)).astype(np.float32)
+    np.testing.assert_array_equal(fused, u / np.float32(255.0))
