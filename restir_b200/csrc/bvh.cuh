@@ -322,11 +322,15 @@ __device__ __forceinline__ int traceBvh(const BvhView& b, V3 o, V3 d, float maxD
 	return hit;
 }
 
-// A visibility (any-hit) ray: traceBvh's stackless walk, or with wave set
-// the warp-lock-step walk of the reference's Vulkan build (same hits).
-__device__ __forceinline__ int traceVisibility(const BvhView& b, V3 o, V3 d, float maxDistance, float& distance, bool wave)
+// A visibility (any-hit) ray: traceBvh's stackless walk, or with kWave the
+// warp-lock-step walk of the reference's Vulkan build (same hits). A template
+// parameter, so that a kernel holds the code it runs and no other: both in one
+// kernel made GI spatial 7,952 instructions instead of 7,184, DI temporal 4,840
+// instead of 4,064.
+template<bool kWave>
+__device__ __forceinline__ int traceVisibility(const BvhView& b, V3 o, V3 d, float maxDistance, float& distance)
 {
-	if (!wave)
+	if (!kWave)
 	{
 		return traceBvh(b, o, d, maxDistance, true, distance, nullptr, 0);
 	}

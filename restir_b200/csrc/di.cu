@@ -191,14 +191,15 @@ struct DiPass
 		return luminance(d + sp);
 	}
 
+	template<bool kWave>
 	__device__ __forceinline__ bool lightVisible(const Surface& surface, V3 point) const
 	{
 		V3 origin = surface.position + surface.surfaceNormal * kDiRayBias();
 		V3 toPoint = point - origin;
 		float pointDistance = length(toPoint);
 		float occluderDistance = 0.0f;
-		return traceVisibility(bvh, origin, toPoint / fmaxf(pointDistance, 0.0001f), pointDistance * 0.999f - kDiRayBias(),
-			occluderDistance, P.wave_visibility > 0.5f) < 0;
+		return traceVisibility<kWave>(bvh, origin, toPoint / fmaxf(pointDistance, 0.0001f), pointDistance * 0.999f - kDiRayBias(),
+			occluderDistance) < 0;
 	}
 
 	__device__ __forceinline__ bool sameSurface(V3 p, V3 n, V3 otherP, V3 otherN, float radius) const
@@ -223,6 +224,7 @@ __device__ __forceinline__ DiPass makeDiPass(const RestirParams& P, const BvhVie
 	return d;
 }
 
+template<bool kWave>
 __global__ void __launch_bounds__(128, RESTIR_DI_TEMPORAL_MIN_BLOCKS) diTemporalKernel(const RestirParams P, BvhView bvh, const float* lights, RestirGBuffer gb,
 	RestirDiReservoirs previous, RestirDiReservoirs out)
 {
@@ -314,7 +316,7 @@ __global__ void __launch_bounds__(128, RESTIR_DI_TEMPORAL_MIN_BLOCKS) diTemporal
 		float previousTarget = 0.0f;
 		if (temporalCount > 0.0f)
 		{
-			if (d.lightVisible(prev, canonicalPoint))
+			if (d.template lightVisible<kWave>(prev, canonicalPoint))
 			{
 				previousTarget = d.lightTarget(prev, canonicalLight, canonicalPoint);
 			}
@@ -343,7 +345,7 @@ __global__ void __launch_bounds__(128, RESTIR_DI_TEMPORAL_MIN_BLOCKS) diTemporal
 	float combinedWeight = chosenTarget > 0.0f ? weightSum / chosenTarget : 0.0f;
 	if (combinedWeight > 0.0f)
 	{
-		if (!d.lightVisible(surface, chosenPoint))
+		if (!d.template lightVisible<kWave>(surface, chosenPoint))
 		{
 			combinedWeight = 0.0f;
 		}
@@ -353,6 +355,7 @@ __global__ void __launch_bounds__(128, RESTIR_DI_TEMPORAL_MIN_BLOCKS) diTemporal
 	storeH4(out.normal, i, v4(surface.normal, canonicalCount + temporalCount));
 }
 
+template<bool kWave>
 __global__ void __launch_bounds__(128, RESTIR_DI_SPATIAL_MIN_BLOCKS) diSpatialKernel(const RestirParams P, BvhView bvh, const float* lights, RestirGBuffer gb,
 	RestirDiReservoirs current, uint16_t* diffuseOut, uint16_t* specularOut)
 {
@@ -418,7 +421,7 @@ __global__ void __launch_bounds__(128, RESTIR_DI_SPATIAL_MIN_BLOCKS) diSpatialKe
 		if (canonicalTarget > 0.0f)
 		{
 			float neighbourTarget = 0.0f;
-			if (d.lightVisible(neighbour, canonicalPoint))
+			if (d.template lightVisible<kWave>(neighbour, canonicalPoint))
 			{
 				neighbourTarget = d.lightTarget(neighbour, canonicalLight, canonicalPoint);
 			}
@@ -458,7 +461,7 @@ __global__ void __launch_bounds__(128, RESTIR_DI_SPATIAL_MIN_BLOCKS) diSpatialKe
 	float combinedWeight = chosenTarget > 0.0f ? weightSum / (totalCount * chosenTarget) : 0.0f;
 	if (combinedWeight > 0.0f && neighbourSelected)
 	{
-		if (!d.lightVisible(surface, chosenPoint))
+		if (!d.template lightVisible<kWave>(surface, chosenPoint))
 		{
 			combinedWeight = 0.0f;
 		}
@@ -490,7 +493,7 @@ extern "C" int restir_di_temporal(const RestirParams* params, const RestirScene*
 		return RESTIR_ERROR_INVALID_ARGUMENT;
 	}
 	dim3 grid((params->width + 15) / 16, (params->height + 7) / 8);
-	diTemporalKernel<<<grid, 128, 0, asStream(stream)>>>(*params, makeBvhView(scene), scene->lights, *gbuffer, *previous, *output);
+	(params->wave_visibility > 0.5f ? diTemporalKernel<true> : diTemporalKernel<false>)<<<grid, 128, 0, asStream(stream)>>>(*params, makeBvhView(scene), scene->lights, *gbuffer, *previous, *output);
 	return launchStatus();
 }
 
@@ -504,7 +507,7 @@ extern "C" int restir_di_spatial(const RestirParams* params, const RestirScene* 
 		return RESTIR_ERROR_INVALID_ARGUMENT;
 	}
 	dim3 grid((params->width + 15) / 16, (params->height + 7) / 8);
-	diSpatialKernel<<<grid, 128, 0, asStream(stream)>>>(*params, makeBvhView(scene), scene->lights, *gbuffer, *current, diffuse,
+	(params->wave_visibility > 0.5f ? diSpatialKernel<true> : diSpatialKernel<false>)<<<grid, 128, 0, asStream(stream)>>>(*params, makeBvhView(scene), scene->lights, *gbuffer, *current, diffuse,
 		specular);
 	return launchStatus();
 }

@@ -162,6 +162,7 @@ __device__ __forceinline__ void boilAndStore(const RestirParams& P, const GiPass
 // cs_restir_temporal.sc:192-296 after the fresh candidates: temporal reuse
 // with pairwise MIS, the boiling filter over the warp's 4x8 group, the
 // reservoir stores. Every lane of the warp must call it (the group sum).
+template<bool kWave>
 __device__ __forceinline__ void temporalReuseAndStore(const RestirParams& P, const GiPass& g, const GiBindings& b, int lane,
 	bool inside, bool working, int px, int py, V3 position, V3 normal, V3 albedo, const GiReservoir& canonical, uint32_t rng)
 {
@@ -214,14 +215,15 @@ __device__ __forceinline__ void temporalReuseAndStore(const RestirParams& P, con
 				GiPass::skipNeighbour(mis);
 				continue;
 			}
-			g.addNeighbour(mis, position, normal, albedo, neighbour, randomSelect);
+			g.template addNeighbour<kWave>(mis, position, normal, albedo, neighbour, randomSelect);
 		}
-		combinedWeight = g.finishPairwiseMis(mis, position, normal, canonical, canonicalWeight, nextRandom(rng));
+		combinedWeight = g.template finishPairwiseMis<kWave>(mis, position, normal, canonical, canonicalWeight, nextRandom(rng));
 	}
 	boilAndStore(P, g, b, lane, inside, working, px, py, position, normal, albedo, canonical, canonicalWeight, previousUv, mis,
 		combinedWeight);
 }
 
+template<bool kWave>
 __global__ void __launch_bounds__(kGiThreads, RESTIR_GI_TEMPORAL_MIN_BLOCKS) giTemporalKernel(const RestirParams P, BvhView bvh,
 	GiBindings b)
 {
@@ -313,9 +315,10 @@ __global__ void __launch_bounds__(kGiThreads, RESTIR_GI_TEMPORAL_MIN_BLOCKS) giT
 		}
 	}
 
-	temporalReuseAndStore(P, g, b, lane, inside, working, px, py, position, normal, albedo, canonical, rng);
+	temporalReuseAndStore<kWave>(P, g, b, lane, inside, working, px, py, position, normal, albedo, canonical, rng);
 }
 
+template<bool kWave>
 __global__ void __launch_bounds__(128, RESTIR_GI_SPATIAL_MIN_BLOCKS) giSpatialKernel(const RestirParams P, BvhView bvh, GiBindings b)
 {
 	const int px = int(blockIdx.x * 16 + threadIdx.x % 16);
@@ -407,10 +410,10 @@ __global__ void __launch_bounds__(128, RESTIR_GI_SPATIAL_MIN_BLOCKS) giSpatialKe
 			GiPass::skipNeighbour(mis);
 			continue;
 		}
-		g.addNeighbour(mis, position, normal, albedo, neighbour, randomSelect);
+		g.template addNeighbour<kWave>(mis, position, normal, albedo, neighbour, randomSelect);
 	}
 
-	const float combinedWeight = g.finishPairwiseMis(mis, position, normal, canonical, canonicalWeight, nextRandom(rng));
+	const float combinedWeight = g.template finishPairwiseMis<kWave>(mis, position, normal, canonical, canonicalWeight, nextRandom(rng));
 	V3 estimate = mis.combined.contribution * combinedWeight;
 	if (P.outlier_clamp > 0.0f)
 	{
@@ -566,6 +569,7 @@ __global__ void __launch_bounds__(128, 8) walkQueueKernel(BvhView bvh, RayQueue 
 	queueWalk<kWide>(bvh, queue, slots);
 }
 
+template<bool kWave>
 __global__ void __launch_bounds__(kGiThreads, RESTIR_GI_TEMPORAL_MIN_BLOCKS) giTemporalShadeKernel(const RestirParams P,
 	BvhView bvh, GiBindings b, CandidateRecords records, RayQueue queue)
 {
@@ -727,7 +731,7 @@ __global__ void __launch_bounds__(kGiThreads, RESTIR_GI_TEMPORAL_MIN_BLOCKS) giT
 			to = mis.combined.position;
 			toId = mis.combined.id;
 		}
-		const bool occluded = test && !g.isVisible(from, fromNormal, to, toId);
+		const bool occluded = test && !g.template isVisible<kWave>(from, fromNormal, to, toId);
 		if (step == candidates + taps)
 		{
 			if (occluded)
@@ -1167,7 +1171,7 @@ extern "C" int restir_gi_temporal(const RestirParams* params, const RestirScene*
 	b.outReceiver = reinterpret_cast<float4*>(output->receiver);
 	b.outNormal = reinterpret_cast<float4*>(output->normal);
 	const int groups = int((params->gi_width + 3) / 4 * ((params->gi_height + 7) / 8));
-	giTemporalKernel<<<(groups + kGiWarps - 1) / kGiWarps, kGiThreads, 0, asStream(stream)>>>(*params, makeBvhView(scene), b);
+	(params->wave_visibility > 0.5f ? giTemporalKernel<true> : giTemporalKernel<false>)<<<(groups + kGiWarps - 1) / kGiWarps, kGiThreads, 0, asStream(stream)>>>(*params, makeBvhView(scene), b);
 	return launchStatus();
 }
 
@@ -1188,7 +1192,7 @@ extern "C" int restir_gi_spatial(const RestirParams* params, const RestirScene* 
 	b.outColor = color;
 	b.outMoments = moments;
 	dim3 grid((params->gi_width + 15) / 16, (params->gi_height + 7) / 8);
-	giSpatialKernel<<<grid, 128, 0, asStream(stream)>>>(*params, makeBvhView(scene), b);
+	(params->wave_visibility > 0.5f ? giSpatialKernel<true> : giSpatialKernel<false>)<<<grid, 128, 0, asStream(stream)>>>(*params, makeBvhView(scene), b);
 	return launchStatus();
 }
 
@@ -1411,7 +1415,7 @@ extern "C" int restir_gi_temporal_wavefront(const RestirParams* params, const Re
 	cudaMemsetAsync(workspace, 0, 3 * sizeof(uint32_t), s);
 	giCandidatesKernel<<<blocks, kGiThreads, 0, s>>>(*params, bvh, b, w.records, w.queue);
 	launchQueueTracer(bvh, w.queue, s);
-	giTemporalShadeKernel<<<blocks, kGiThreads, 0, s>>>(*params, bvh, b, w.records, w.queue);
+	(params->wave_visibility > 0.5f ? giTemporalShadeKernel<true> : giTemporalShadeKernel<false>)<<<blocks, kGiThreads, 0, s>>>(*params, bvh, b, w.records, w.queue);
 	return launchStatus();
 }
 
@@ -1615,7 +1619,7 @@ extern "C" int restir_gi_temporal_shade(const RestirParams* params, const Restir
 	b.outReceiver = reinterpret_cast<float4*>(output->receiver);
 	b.outNormal = reinterpret_cast<float4*>(output->normal);
 	const int groups = int((params->gi_width + 3) / 4 * ((params->gi_height + 7) / 8));
-	giTemporalShadeKernel<<<(groups + kGiWarps - 1) / kGiWarps, kGiThreads, 0, asStream(stream)>>>(*params, makeBvhView(scene),
+	(params->wave_visibility > 0.5f ? giTemporalShadeKernel<true> : giTemporalShadeKernel<false>)<<<(groups + kGiWarps - 1) / kGiWarps, kGiThreads, 0, asStream(stream)>>>(*params, makeBvhView(scene),
 		b, r, q);
 	return launchStatus();
 }
@@ -1996,7 +2000,7 @@ extern "C" int restir_gi_temporal_cached(const RestirParams* params, const Resti
 	}
 	b.cache = w.cache.values;
 	b.cacheNeighbourBase = int(candidates);
-	giTemporalShadeKernel<<<blocks, kGiThreads, 0, s>>>(*params, bvh, b, w.records, w.queue);
+	(params->wave_visibility > 0.5f ? giTemporalShadeKernel<true> : giTemporalShadeKernel<false>)<<<blocks, kGiThreads, 0, s>>>(*params, bvh, b, w.records, w.queue);
 	return launchStatus();
 }
 
@@ -2038,7 +2042,7 @@ extern "C" int restir_gi_spatial_cached(const RestirParams* params, const Restir
 	b.cache = w.cache.values;
 	b.cacheNeighbourBase = 0;
 	dim3 grid((params->gi_width + 15) / 16, (params->gi_height + 7) / 8);
-	giSpatialKernel<<<grid, 128, 0, s>>>(*params, bvh, b);
+	(params->wave_visibility > 0.5f ? giSpatialKernel<true> : giSpatialKernel<false>)<<<grid, 128, 0, s>>>(*params, bvh, b);
 	return launchStatus();
 }
 

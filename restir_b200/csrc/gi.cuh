@@ -575,6 +575,7 @@ struct GiPass
 		return receiverCosine > 0.0f && sampleCosine > 0.0f ? receiverCosine * sampleCosine / distanceSquared : 0.0f;
 	}
 
+	template<bool kWave>
 	__device__ inline bool isVisible(V3 receiverPosition, V3 receiverNormal, V3 samplePosition, float sampleId) const
 	{
 		V3 origin = receiverPosition + receiverNormal * kRayBias();
@@ -588,8 +589,8 @@ struct GiPass
 		if (bvhRay)
 		{
 			float occluderDistance = 0.0f;
-			return traceVisibility(bvh, origin, direction, sky ? kMaxBvhRayDistance() : sampleDistance - kRayBias(),
-				occluderDistance, P.wave_visibility > 0.5f) < 0;
+			return traceVisibility<kWave>(bvh, origin, direction, sky ? kMaxBvhRayDistance() : sampleDistance - kRayBias(),
+				occluderDistance) < 0;
 		}
 		if (sky)
 		{
@@ -734,13 +735,14 @@ struct GiPass
 		}
 	}
 
+	template<bool kWave>
 	__device__ inline void addNeighbour(PairwiseMis& mis, V3 p, V3 n, V3 albedo, const NeighbourReservoir& nb, float random) const
 	{
 		float neighbourGeometry;
 		bool occluded = false;
 		if (neighbourBegin(mis, nb, neighbourGeometry))
 		{
-			occluded = !isVisible(nb.receiverPosition, nb.receiverNormal, mis.canonicalPosition, mis.canonicalId);
+			occluded = !isVisible<kWave>(nb.receiverPosition, nb.receiverNormal, mis.canonicalPosition, mis.canonicalId);
 		}
 		neighbourShare(mis, nb, neighbourGeometry, occluded);
 		V3 contribution = v3s(0.0f);
@@ -774,13 +776,14 @@ struct GiPass
 		return combinedWeight > 0.0f && mis.neighbourSelected;
 	}
 
+	template<bool kWave>
 	__device__ inline float finishPairwiseMis(PairwiseMis& mis, V3 p, V3 n, const GiReservoir& canonical, float canonicalWeight,
 		float random) const
 	{
 		float combinedWeight;
 		if (finishBegin(mis, canonical, canonicalWeight, random, combinedWeight))
 		{
-			if (!isVisible(p, n, mis.combined.position, mis.combined.id))
+			if (!isVisible<kWave>(p, n, mis.combined.position, mis.combined.id))
 			{
 				combinedWeight = 0.0f;
 			}

@@ -121,7 +121,7 @@ __global__ void __launch_bounds__(kTraceBlock) traceKernel(BvhView bvh, RayArray
 	}
 	else if (kKind == RESTIR_TRACE_ANY_WAVE)
 	{
-		r.hit = traceVisibility(bvh, r.o, r.d, length, r.distance, true);
+		r.hit = traceVisibility<true>(bvh, r.o, r.d, length, r.distance);
 	}
 	else
 	{
