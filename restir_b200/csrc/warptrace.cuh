@@ -9,117 +9,12 @@
 // leaf waits for others, and four lanes test each waiting leaf, one triangle a
 // lane.
 //
-// A node is read with one 256-bit load where the buffer starts on 32 bytes
-// (kWide; the layout's nodes are 32 bytes), else with two of 128 bits, and
-// its slab test runs on packed pairs of floats (add and mul.rn.f32x2 round each
-// half as the scalar operations do).
 #pragma once
 
 #include "bvh.cuh"
 
 namespace restir
 {
-
-// --- packed pairs --------------------------------------------------------------
-
-typedef unsigned long long F2;
-
-__device__ __forceinline__ F2 pack2(float a, float b)
-{
-	F2 r;
-	asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-	return r;
-}
-
-__device__ __forceinline__ void unpack2(F2 v, float& a, float& b)
-{
-	asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-
-__device__ __forceinline__ F2 add2(F2 a, F2 b)
-{
-	F2 r;
-	asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-	return r;
-}
-
-__device__ __forceinline__ F2 mul2(F2 a, F2 b)
-{
-	F2 r;
-	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-	return r;
-}
-
-// --- nodes ---------------------------------------------------------------------
-
-// A node's 32 bytes: (min.xy) (min.z, a) (max.xy) (max.z, b).
-struct NodeRow
-{
-	F2 lo, loA, hi, hiB;
-};
-
-template<bool kWide>
-__device__ __forceinline__ NodeRow loadNode(const BvhView& b, int node)
-{
-	NodeRow n;
-	if (!checkedIndex(uint32_t(node) * 2u + 1u, uint32_t(b.rowCount)))
-	{
-		n.lo = n.loA = n.hi = n.hiB = 0ull;
-		return n;
-	}
-	const float4* row = b.rows + size_t(node) * 2;
-	if (kWide)
-	{
-		asm("ld.global.nc.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(n.lo), "=l"(n.loA), "=l"(n.hi), "=l"(n.hiB) : "l"(row));
-	}
-	else
-	{
-		asm("ld.global.nc.v2.b64 {%0, %1}, [%2];" : "=l"(n.lo), "=l"(n.loA) : "l"(row));
-		asm("ld.global.nc.v2.b64 {%0, %1}, [%2];" : "=l"(n.hi), "=l"(n.hiB) : "l"(row + 1));
-	}
-	return n;
-}
-
-// A ray as the slab test takes it: the negated origin and the inverse direction.
-struct SlabRay
-{
-	F2 negXY, invXY;
-	float negZ, invZ;
-};
-
-__device__ __forceinline__ SlabRay slabRay(V3 o, V3 d)
-{
-	const V3 inv = bvhInverseDirection(d);
-	SlabRay r;
-	r.negXY = pack2(-o.x, -o.y);
-	r.invXY = pack2(inv.x, inv.y);
-	r.negZ = -o.z;
-	r.invZ = inv.z;
-	return r;
-}
-
-__device__ __forceinline__ V3 slabOrigin(const SlabRay& r)
-{
-	float x, y;
-	unpack2(r.negXY, x, y);
-	return v3(-x, -y, -r.negZ);
-}
-
-// intersectBox (bvh.sh:32-41); a and b are the node's two words.
-__device__ __forceinline__ float slabEnter(const SlabRay& r, const NodeRow& n, float maxDistance, float& a, float& b)
-{
-	float loZ, hiZ;
-	unpack2(n.loA, loZ, a);
-	unpack2(n.hiB, hiZ, b);
-	float t0x, t0y, t1x, t1y;
-	unpack2(mul2(add2(n.lo, r.negXY), r.invXY), t0x, t0y);
-	unpack2(mul2(add2(n.hi, r.negXY), r.invXY), t1x, t1y);
-	const float t0z = (loZ + r.negZ) * r.invZ;
-	const float t1z = (hiZ + r.negZ) * r.invZ;
-	const float enter = fmaxf(fmaxf(fminf(t0x, t1x), fminf(t0y, t1y)), fmaxf(fminf(t0z, t1z), 0.0f));
-	const float leave = fminf(fminf(fmaxf(t0x, t1x), fmaxf(t0y, t1y)), fminf(fmaxf(t0z, t1z), maxDistance));
-	return enter <= leave ? enter : -1.0f;
-}
 
 // --- leaves --------------------------------------------------------------------
 
@@ -236,10 +131,10 @@ __device__ __forceinline__ bool testLeaves(const BvhView& b, LeafSlots& slots, b
 
 // --- rays ----------------------------------------------------------------------
 //
-// traceNearest and traceWalks trace rays until their source has no more. Every
+// traceNearest, traceLaneWalks and traceGroupWalks trace rays until their source has no more. Every
 // lane of the warp calls them. A source gives
-//   take(idle, more, r): called by the whole warp; an idle lane (traceWalks: the
-//     four lanes of an idle group) gets a ray in r, r.index -1 when there is
+//   take(idle, more, r): called by the whole warp; an idle lane (traceGroupWalks:
+//     the four lanes of an idle group) gets a ray in r, r.index -1 when there is
 //     none for it, and more is cleared when there are none left;
 //   store(r): the ray's hit and distance;
 //   kCount: the kind of ray to count (-1: a ray counted before).
@@ -296,7 +191,7 @@ struct NearestStorage
 };
 
 // Nearest hits with the short stack (bvh.sh:216-295), a ray per lane. A ray
-// whose stack dropped entries is stored marked (markedHit): traceWalks finishes
+// whose stack dropped entries is stored marked (markedHit): a walk finishes
 // it. In one loop with the short stack, the re-walk would make the two halves
 // of a warp wait for each other (18% of random rays in the 1M-triangle city
 // drop entries, and their re-walk visits 142 nodes after 53). Bound by the L1's
@@ -460,33 +355,22 @@ __device__ __forceinline__ void traceNearest(const BvhView& b, Source& source, N
 	}
 }
 
-// The warp leaves its stepping loop when this share (1 / n) of its groups with a
-// ray have stopped, and stores and takes rays when so many groups have ended.
-#ifndef RESTIR_WALK_SHARE
-#	define RESTIR_WALK_SHARE 3
-#endif
-#ifndef RESTIR_WALK_REFILL
-#	define RESTIR_WALK_REFILL 1
-#endif
-
-// The stackless walk (bvh.sh:140-174; kAny: to the first leaf with a hit),
-// kLanes lanes a ray. The layout is depth first and a walk goes on to the next
-// node or over a subtree, so four consecutive nodes hold 2.3 of its visits on
-// average (1M-triangle city; two hold 1.65, eight 2.7): with kLanes 4 the lanes
-// of a group read and test one each (128 consecutive bytes), and the group
-// follows the walk through the results. That divides a walk's chain of
-// dependent loads by 2.3, for launches that its latency bounds: the specular
-// rays of a 1283x717 frame take 0.51 ms, 0.87 ms in the one-lane loop it
-// replaces (the longest walks, up to 2,048 visits, end last); where rays
-// abound, a ray per lane (kLanes 1) does more with the same instructions.
-template<bool kAny, bool kWide, int kLanes, typename Source>
-__device__ __forceinline__ void traceWalks(const BvhView& b, Source& source, LeafSlots& slots)
+// The stackless walk (bvh.sh:140-174; kAny: to the first leaf with a hit), four
+// lanes a ray. The layout is depth first and a walk goes on to the next node
+// or over a subtree, so four consecutive nodes hold 2.3 of its visits on
+// average (1M-triangle city; two hold 1.65, eight 2.7): the lanes of a group
+// read and test one each (128 consecutive bytes), and the group follows the
+// walk through the results. That divides a walk's chain of dependent loads by
+// 2.3, for launches that its latency bounds (the longest walks, up to 2,048
+// visits, end last): the specular rays of a 1283x717 frame take 0.51 ms, with a
+// ray per lane 0.62 ms, 0.87 ms in the one-lane loop with unshared leaves.
+template<bool kAny, bool kWide, typename Source>
+__device__ __forceinline__ void traceGroupWalks(const BvhView& b, Source& source)
 {
 	const int lane = int(threadIdx.x & 31u);
-	const int group = lane & ~(kLanes - 1);
-	const int sub = lane & (kLanes - 1);
+	const int group = lane & 28;
+	const int sub = lane & 3;
 	constexpr unsigned kAll = 0xffffffffu;
-	constexpr unsigned kGroup = (1u << kLanes) - 1u;
 	constexpr int kAtLeaf = 0x7fffffff;
 	Ray r = {};
 	r.index = -1;
@@ -502,8 +386,7 @@ __device__ __forceinline__ void traceWalks(const BvhView& b, Source& source, Lea
 	for (;;)
 	{
 		// Rays that have ended are stored, and groups without one take the next.
-		const unsigned ended = __ballot_sync(kAll, !go && !waiting && (r.index >= 0 || more));
-		if (__popc(ended) >= RESTIR_WALK_REFILL * kLanes || (ended != 0u && __all_sync(kAll, !go && !waiting)))
+		if (__any_sync(kAll, !go && !waiting && (r.index >= 0 || more)))
 		{
 			if (!go && !waiting && r.index >= 0)
 			{
@@ -537,7 +420,7 @@ __device__ __forceinline__ void traceWalks(const BvhView& b, Source& source, Lea
 			}
 			continue;
 		}
-		const int limit = rays - max(rays / RESTIR_WALK_SHARE, kLanes);
+		const int limit = rays - max(rays / 3, 4);
 		do
 		{
 			const int last = b.nodeCount - node;  // the walk ends at this lane
@@ -552,38 +435,24 @@ __device__ __forceinline__ void traceWalks(const BvhView& b, Source& source, Lea
 			// leaf it enters, the end.
 			const bool turned = leaf == pass || sub >= last;
 			const int away = leaf ? kAtLeaf : int(-w) - 1 - node;   // the skip target, from the first node
-			int at, visits, target;
-			if (kLanes == 1)
+			const unsigned turns = __ballot_sync(kAll, turned) >> group & 15u;
+			int at = turns != 0u ? __ffs(turns) - 1 : 4;
+			int visits = at;
+			// A subtree of three nodes missed at the first lane ends before the last.
+			if (__shfl_sync(kAll, away, group) == 3 && at == 0)
 			{
-				at = turned ? 0 : 1;
-				visits = at;
-				target = away;
+				at = (turns & 8u) != 0u ? 3 : 4;
+				visits = at - 2;
 			}
-			else
-			{
-				const unsigned turns = __ballot_sync(kAll, turned) >> group & kGroup;
-				at = turns != 0u ? __ffs(turns) - 1 : kLanes;
-				visits = at;
-				if (kLanes == 4)
-				{
-					// A subtree of three nodes missed at the first lane ends before the last.
-					const int over = __shfl_sync(kAll, away, group);
-					if (over == 3 && at == 0)
-					{
-						at = (turns & 8u) != 0u ? 3 : 4;
-						visits = at - 2;
-					}
-				}
-				target = __shfl_sync(kAll, away, group | (at & (kLanes - 1)));
-			}
+			const int target = __shfl_sync(kAll, away, group | (at & 3));
 			if (go)
 			{
 				const bool end = at >= last;
-				const bool missed = at < kLanes && target != kAtLeaf;
+				const bool missed = at < 4 && target != kAtLeaf;
 				turn = at;
-				waiting = !end && at < kLanes && target == kAtLeaf;
+				waiting = !end && at < 4 && target == kAtLeaf;
 				step += visits + (missed && !end ? 1 : 0);
-				node += waiting ? 0 : (missed ? target : kLanes);
+				node += waiting ? 0 : (missed ? target : 4);
 				go = !end && !waiting && node < b.nodeCount;
 				if (step >= kBvhMaxSteps)
 				{
@@ -599,52 +468,29 @@ __device__ __forceinline__ void traceWalks(const BvhView& b, Source& source, Lea
 		} while (__popc(__ballot_sync(kAll, go)) > limit);
 		if (__any_sync(kAll, waiting))
 		{
-			int count;
-			bool tested;
-			if (kLanes == 4)
+			const int first = int(__shfl_sync(kAll, a, group | (turn & 3)));
+			const float leafWord = __shfl_sync(kAll, w, group | (turn & 3));
+			const int count = waiting ? int(leafWord) : 0;
+			int t = 0;
+			do
 			{
-				const int first = int(__shfl_sync(kAll, a, group | (turn & 3)));
-				const float leafWord = __shfl_sync(kAll, w, group | (turn & 3));
-				count = waiting ? int(leafWord) : 0;
-				int t = 0;
-				do
+				float h = -1.0f;
+				if (t + sub < count)
 				{
-					float h = -1.0f;
-					if (t + sub < count)
-					{
-						h = leafTriangle<kWide>(b, first + t + sub, r.o, r.d);
-					}
-					const unsigned key = h > 0.0f && h < r.distance ? __float_as_uint(h) : kAll;
-					unsigned nearest = min(key, __shfl_xor_sync(kAll, key, 1));
-					nearest = min(nearest, __shfl_xor_sync(kAll, nearest, 2));
-					const unsigned winners = __ballot_sync(kAll, key == nearest && key != kAll) >> group & 15u;
-					if (winners != 0u)
-					{
-						r.distance = __uint_as_float(nearest);
-						r.hit = first + t + __ffs(winners) - 1;
-					}
-					t += 4;
-				} while (__any_sync(kAll, t < count));
-				tested = waiting;
-			}
-			else
-			{
-				int first = int(a);
-				count = int(w);
-				if (kLanes == 2)
-				{
-					first = __shfl_sync(kAll, first, group | (turn & 1));
-					count = __shfl_sync(kAll, count, group | (turn & 1));
+					h = leafTriangle<kWide>(b, first + t + sub, r.o, r.d);
 				}
-				tested = testLeaves<kWide>(b, slots, waiting && sub == 0, r.o, r.d, first, count, r.distance, r.hit);
-				if (kLanes == 2)
+				const unsigned key = h > 0.0f && h < r.distance ? __float_as_uint(h) : kAll;
+				unsigned nearest = min(key, __shfl_xor_sync(kAll, key, 1));
+				nearest = min(nearest, __shfl_xor_sync(kAll, nearest, 2));
+				const unsigned winners = __ballot_sync(kAll, key == nearest && key != kAll) >> group & 15u;
+				if (winners != 0u)
 				{
-					tested = __shfl_sync(kAll, int(tested), group) != 0;
-					r.distance = __shfl_sync(kAll, r.distance, group);
-					r.hit = __shfl_sync(kAll, r.hit, group);
+					r.distance = __uint_as_float(nearest);
+					r.hit = first + t + __ffs(winners) - 1;
 				}
-			}
-			if (tested)
+				t += 4;
+			} while (__any_sync(kAll, t < count));
+			if (waiting)
 			{
 				triangles += uint32_t(count);
 				waiting = false;
@@ -656,10 +502,92 @@ __device__ __forceinline__ void traceWalks(const BvhView& b, Source& source, Lea
 	}
 }
 
-// Whether a scene's nodes can be read 32 bytes at a time.
-__host__ inline bool wideRows(const BvhView& b)
+// The same with a ray per lane and the leaves tested together, for launches with
+// more rays than lanes: 1M any-hit rays in the city take 0.39 ms, 0.65 ms with
+// unshared leaves (6 of 32 lanes active there, 21 here) and 0.74 ms with four
+// lanes a ray; half of its instructions take rays and test leaves.
+template<bool kAny, bool kWide, typename Source>
+__device__ __forceinline__ void traceLaneWalks(const BvhView& b, Source& source, LeafSlots& slots)
 {
-	return (reinterpret_cast<uintptr_t>(b.rows) & 31u) == 0u;
+	constexpr unsigned kAll = 0xffffffffu;
+	Ray r = {};
+	r.index = -1;
+	SlabRay slab = {};
+	int node = 0;
+	int step = 0;
+	uint32_t triangles = 0;
+	bool go = false;
+	bool waiting = false;
+	float a = 0.0f, w = 0.0f;
+	bool more = true;
+	for (;;)
+	{
+		if (__any_sync(kAll, !go && !waiting && (r.index >= 0 || more)))
+		{
+			if (!go && !waiting && r.index >= 0)
+			{
+				if (step >= kBvhMaxSteps && !(kAny && r.hit >= 0))
+				{
+					reportTruncatedRay();
+				}
+				countWork(Source::kCount, uint32_t(step), triangles);
+				source.store(r);
+				r.index = -1;
+			}
+			if (more)
+			{
+				const bool take = r.index < 0;
+				source.take(take, more, r);
+				if (take && r.index >= 0)
+				{
+					slab = slabRay(r.o, r.d);
+					node = 0;
+					step = 0;
+					triangles = 0;
+					go = b.available();
+				}
+			}
+		}
+		const int rays = __popc(__ballot_sync(kAll, r.index >= 0));
+		if (rays == 0)
+		{
+			if (!more)
+			{
+				break;
+			}
+			continue;
+		}
+		const int limit = rays - max(rays / 3, 1);
+		do
+		{
+#pragma unroll
+			for (int k = 0; k < 4; ++k)
+			{
+				if (go)
+				{
+					const bool pass = slabEnter(slab, loadNode<kWide>(b, node), r.distance, a, w) >= 0.0f;
+					const bool leaf = w >= 0.0f;
+					waiting = pass && leaf;
+					const int next = pass || leaf ? node + 1 : int(-w) - 1;
+					node = waiting ? node : next;
+					step += waiting ? 0 : 1;
+					go = !waiting && node < b.nodeCount && step < kBvhMaxSteps;
+				}
+			}
+		} while (__popc(__ballot_sync(kAll, go)) > limit);
+		if (__any_sync(kAll, waiting))
+		{
+			const int count = int(w);
+			if (testLeaves<kWide>(b, slots, waiting, r.o, r.d, int(a), count, r.distance, r.hit))
+			{
+				triangles += uint32_t(count);
+				waiting = false;
+				++step;
+				++node;
+				go = !(kAny && r.hit >= 0) && node < b.nodeCount && step < kBvhMaxSteps;
+			}
+		}
+	}
 }
 
 } // namespace restir

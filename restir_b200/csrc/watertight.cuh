@@ -92,10 +92,11 @@ __device__ __forceinline__ float intersectWatertight(const WatertightRay& r, V3 
 
 // Nearest watertight hit in (0, distance], ties to the lower triangle index,
 // with conservative box tests.
+template<bool kWide>
 __device__ inline int traceWatertight(const BvhView& b, V3 o, V3 d, float& distance)
 {
 	const WatertightRay ray = makeWatertightRay(o, d);
-	return traceNearestFirst(b, o, d, distance, true,
+	return traceNearestFirst<kWide, false, true>(b, o, d, distance,
 		[&](int t, float tmax) { return intersectWatertight(ray, b.vertex(t, 0), b.vertex(t, 1), b.vertex(t, 2), tmax); },
 		[](int) { return true; });
 }

@@ -117,7 +117,7 @@ struct QueueSource
 };
 
 // The marked rays (markedHit) among the first `end` of a ray set: a source for
-// traceWalks. The warp looks through 32 consecutive rays at a time, the next
+// the walks. The warp looks through 32 consecutive rays at a time, the next
 // ones no warp has claimed (claimed), or the next of its own part (null).
 template<int kLanes>
 struct MarkedSource
@@ -185,15 +185,22 @@ __device__ __forceinline__ void queueNearest(const BvhView& b, const RayQueue& q
 template<bool kWide>
 __device__ __forceinline__ void queueRewalk(const BvhView& b, const RayQueue& q, LeafSlots* slots)
 {
-	MarkedSource<4> source{ { q.rays, q.hitTriangle, q.hitDistance }, 0u, queuedRays(q), q.claimed + 1 };
-	traceWalks<false, kWide, 4>(b, source, slots[threadIdx.x >> 5]);
+	MarkedSource<1> source{ { q.rays, q.hitTriangle, q.hitDistance }, 0u, queuedRays(q), q.claimed + 1 };
+	traceLaneWalks<false, kWide>(b, source, slots[threadIdx.x >> 5]);
 }
 
-template<bool kWide>
+template<bool kWide, int kLanes>
 __device__ __forceinline__ void queueWalk(const BvhView& b, const RayQueue& q, LeafSlots* slots)
 {
-	QueueSource<RESTIR_COUNT_ANY, 4> source(q);
-	traceWalks<false, kWide, 4>(b, source, slots[threadIdx.x >> 5]);
+	QueueSource<RESTIR_COUNT_ANY, kLanes> source(q);
+	if constexpr (kLanes == 1)
+	{
+		traceLaneWalks<false, kWide>(b, source, slots[threadIdx.x >> 5]);
+	}
+	else
+	{
+		traceGroupWalks<false, kWide>(b, source);
+	}
 }
 
 } // namespace restir
