@@ -82,6 +82,14 @@ RN_HD float rn_round(float x)
 	return x < 0.0f ? -r : r;
 }
 
+/* The same as an integer (its float is rn_round's value; a conversion less
+ * where both are wanted). */
+RN_HD int rn_round_int(float x)
+{
+	int i = (int)((x < 0.0f ? -x : x) + 0.5f);
+	return x < 0.0f ? -i : i;
+}
+
 /* pi / 2 split into three floats (Cody and Waite): the first two have few
  * significant bits, so k times them is exact for |k| < 2^15. */
 #define RN_PIO2_HI 1.5703125f
@@ -141,22 +149,29 @@ RN_HD float rn_cos(float x)
 
 /* e^x. Reduction x = k ln2 + r with |r| <= ln2/2, Taylor series of e^r to
  * r^8, then scaling by 2^k in two exact steps (one rounding into the
- * denormal range). */
+ * denormal range). Where e^x is a normal number the scaling is exact, and
+ * adding k to the exponent is the same (a third of the instructions went to
+ * the two products and the range tests). */
 RN_HD float rn_exp(float x)
 {
-	if (x != x)
+	int normal = x > -86.0f && x < 86.0f;
+	if (!normal)
 	{
-		return x;
+		if (x != x)
+		{
+			return x;
+		}
+		if (x > 88.72283935546875f)
+		{
+			return rn_bits_float(0x7f800000u);
+		}
+		if (x < -103.97208f)
+		{
+			return 0.0f;
+		}
 	}
-	if (x > 88.72283935546875f)
-	{
-		return rn_bits_float(0x7f800000u);
-	}
-	if (x < -103.97208f)
-	{
-		return 0.0f;
-	}
-	float k = rn_round(x * RN_LOG2E);
+	int n = rn_round_int(x * RN_LOG2E);
+	float k = (float)n;
 	float r = x - k * RN_LN2_HI;
 	r = r - k * RN_LN2_LO;
 	float p = 2.4801587301587302e-05f;       /* 1/8! */
@@ -168,7 +183,10 @@ RN_HD float rn_exp(float x)
 	p = p * r + 0.5f;
 	p = p * r + 1.0f;
 	p = p * r + 1.0f;
-	int n = (int)k;
+	if (normal)
+	{
+		return rn_bits_float(rn_float_bits(p) + ((uint32_t)n << 23));
+	}
 	int n1 = n / 2;
 	int n2 = n - n1;
 	return (p * rn_exp2i(n1)) * rn_exp2i(n2);
@@ -233,9 +251,13 @@ RN_HD float rn_exp2(float x)
 	{
 		return 0.0f;
 	}
-	float k = rn_round(x);
-	float r = x - k;
-	int n = (int)k;
+	int n = rn_round_int(x);
+	float r = x - (float)n;
+	if (x > -120.0f && x < 120.0f)
+	{
+		/* Exact, as in rn_exp. */
+		return rn_bits_float(rn_float_bits(rn_exp(r * RN_LN2)) + ((uint32_t)n << 23));
+	}
 	int n1 = n / 2;
 	int n2 = n - n1;
 	return (rn_exp(r * RN_LN2) * rn_exp2i(n1)) * rn_exp2i(n2);
