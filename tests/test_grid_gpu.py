@@ -50,3 +50,26 @@ def test_grid_insert(scene, size, table, mode):
             np.testing.assert_array_equal(np.sort(dentries), np.sort(entries))
     # No probe sequence ran out.
     assert rb.status_flags() & 2 == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("capacity", [1, 5, 32, 77])
+@pytest.mark.parametrize("cell", [1.0, 40.0])
+def test_grid_insert_crowded_cells(capacity, cell):
+    """Lists that overflow, at capacities with and without a multiple of four: each
+    cell keeps its lowest pixel indices in order wherever their insertion starts."""
+    setup = make_scene(rb.SCENE_CORNELL, 0)
+    params, _ = params_for(setup, 253, 131, grid_table_size=1 << 12, grid_mode=rb.GRID_DETERMINISTIC, gi_divisor=1)
+    params.grid_cell_capacity = capacity
+    params.grid_min_cell *= cell
+    gb = host_gbuffer(253, 131)
+    ob.load().oracle_gbuffer_primary(params, setup.host_scene(), gbuffer_struct(gb))
+    host, dev = run_grid(setup, params, gb)
+    hc = grid_cells(host, 1 << 12, capacity)
+    dc = grid_cells(dev, 1 << 12, capacity)
+    assert set(hc) == set(dc)
+    assert max(count for count, _ in hc.values()) > capacity or cell == 1.0
+    for key, (count, entries) in hc.items():
+        assert dc[key][0] == count
+        np.testing.assert_array_equal(dc[key][1], entries)
+    rb.status_flags()
