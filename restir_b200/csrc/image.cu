@@ -55,8 +55,8 @@ __device__ __forceinline__ float geometryWeight(float planeScale, V3 p, V3 n, fl
 
 // The spatial estimate of the variance, of the pixels with less than four
 // frames of history: a block that has one reads its 22x14 texels to shared
-// memory once (each of 49 taps fetched 40 bytes and normalised a normal: the
-// denoiser's inputs at 960x540, a third of them short, 0.136 ms).
+// memory once. With 49 taps that each fetched 40 bytes and normalised a normal
+// it took 0.135 ms on 960x540 pixels, a third of them short; now 0.069 ms.
 constexpr int kVarianceTileW = kFilterW + 6, kVarianceTileH = kFilterH + 6;
 
 __global__ void __launch_bounds__(128) varianceKernel(const RestirParams P, const uint16_t* __restrict__ color,
@@ -271,7 +271,12 @@ __device__ __forceinline__ V3 compositeSpecularAlbedo(V3 f0, float roughness, fl
 
 // fs_composite.sc:48-143 with the final view's options; the indirect
 // specular when a specular target is given.
-__global__ void __launch_bounds__(128) compositeKernel(const RestirParams P, RestirGBuffer gb, const float* __restrict__ atlas,
+// Bound by the latency of its taps and divisions: eight blocks a SM (64
+// registers, 40 bytes spilled) where 94 registers left five: 0.201 -> 0.145 ms
+// at 1920x1080, 0.094 -> 0.073 ms at 1280x720, 0.0116 -> 0.0125 at 256x256, where
+// three and a half blocks a SM are all there are; ten blocks gain 0.007 ms more
+// there and lose 0.002 here.
+__global__ void __launch_bounds__(128, 8) compositeKernel(const RestirParams P, RestirGBuffer gb, const float* __restrict__ atlas,
 	const uint16_t* __restrict__ gi, const uint16_t* __restrict__ diDiffuse, const uint16_t* __restrict__ diSpecular,
 	const uint16_t* __restrict__ specularTarget, uint16_t* hdr)
 {
