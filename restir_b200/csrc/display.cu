@@ -2,9 +2,9 @@
 // exposure (cs_exposure.sc:30-82), TAA (fs_taa.sc:38-172) and tone mapping
 // (fs_tonemap.sc:105-162, tonemap.sh:17-122).
 //
-// All three are HBM-bound image work. The exposure reduction reads 4,096
-// texels with one block. TAA and tone mapping run fused, one thread per pixel
-// in 16x8 tiles: a pixel's tone mapping needs only that pixel's TAA output,
+// The exposure reduction reads 4,096 texels with one block. TAA and tone
+// mapping run fused, one thread per pixel in 32x16 tiles: a pixel's tone
+// mapping needs only that pixel's TAA output,
 // so the fused kernel writes the TAA target (the next frame's history) and
 // tone-maps the same value, rounded to half as the target stores it, without
 // reading it back. The 3x3 neighbourhood and the history's 5 bilinear
@@ -18,11 +18,14 @@ namespace restir
 namespace
 {
 
-// Blocks per SM the display kernel is compiled for: a register cap of 64 (8 blocks
-// of 128 threads) runs the fused TAA + AgX launch at 1080p in 0.21 ms against
-// 0.27 ms uncapped (109 registers).
+// Blocks per SM the display kernel is compiled for: 3 of 512 threads, 40 registers.
+// The kernel is bound by its instructions, some 2,000 a pixel passed once from
+// start to end, and by fetching them: large blocks, whose barrier keeps 16 warps
+// in the same part of them, took 0.263 ms at 2560x1440 (0.049 at 960x540) where
+// blocks of 128 and of 256 threads took 0.312 and 0.302 (0.058, 0.056), and 2
+// blocks of 512 0.291 (0.053).
 #ifndef RESTIR_DISPLAY_MIN_BLOCKS
-#define RESTIR_DISPLAY_MIN_BLOCKS 8
+#define RESTIR_DISPLAY_MIN_BLOCKS 3
 #endif
 
 constexpr int kModeTaa = 1;      // TAA into taaOut
@@ -126,35 +129,52 @@ __device__ __forceinline__ bool anyNan(V3 v)
 	return v.x != v.x || v.y != v.y || v.z != v.z;
 }
 
-// A tile of 16x8 pixels with a one-texel border: each texel's compressed
-// YCoCg colour and depth, computed once for the 9 pixels that read it.
-constexpr int kTileW = 16, kTileH = 8;
+// A tile of 32x16 pixels with a one-texel border: each texel's compressed
+// YCoCg colour and depth, computed once for the 9 pixels that read it (1.2
+// texels a pixel; 1.4 in a tile of 16x8).
+constexpr int kTileW = 32, kTileH = 16;
 constexpr int kHaloW = kTileW + 2, kHaloH = kTileH + 2;
 
-// Fills the tile of the block at (x0, y0). A neighbour's texture coordinate
-// uv + (dx, dy) / size point-samples texel clamp(x + dx, 0, W - 1) exactly
-// for sizes up to 16384: the float sum is within 0.01 of the texel centre.
-__device__ __forceinline__ void loadNeighbourhood(float4* tile, const uint16_t* __restrict__ hdr,
-	const float* __restrict__ depth, int W, int H, int x0, int y0)
+// The texel (tx, ty) of the tile. A neighbour's
+// texture coordinate uv + (dx, dy) / size point-samples texel
+// clamp(x + dx, 0, W - 1) exactly for sizes up to 16384: the float sum is
+// within 0.01 of the texel centre.
+__device__ __forceinline__ void storeTexel(float4* tile, int tx, int ty, V3 compressed, float depth)
 {
-	for (int k = int(threadIdx.x); k < kHaloW * kHaloH; k += int(blockDim.x))
+	const V3 c = toYCoCg(compressed);
+	tile[ty * kHaloW + tx] = make_float4(c.x, c.y, c.z, depth);
+}
+
+// Fills the tile of the block at (x0, y0): each thread its own pixel's texel
+// (its colour in current, compressed in compressed), the first ones the border's.
+__device__ __forceinline__ void loadNeighbourhood(float4* tile, const uint16_t* __restrict__ hdr,
+	const float* __restrict__ depth, int W, int H, int x0, int y0, int lx, int ly, V4& current, V3& compressed)
+{
+	constexpr int kBorder = 2 * kHaloW + 2 * kTileH;
+	static_assert(kBorder <= kTileW * kTileH, "a texel of the border per thread");
+	const int own = min(y0 + ly, H - 1) * W + min(x0 + lx, W - 1);
+	current = loadH4(hdr, own);
+	compressed = compress(current.xyz());
+	storeTexel(tile, lx + 1, ly + 1, compressed, loadF1(depth, own));
+	const int k = int(threadIdx.x);
+	if (k < kBorder)
 	{
-		const int gx = min(max(x0 + k % kHaloW - 1, 0), W - 1);
-		const int gy = min(max(y0 + k / kHaloW - 1, 0), H - 1);
-		const int t = gy * W + gx;
-		const V3 c = toYCoCg(compress(loadH3(hdr, t)));
-		tile[k] = make_float4(c.x, c.y, c.z, loadF1(depth, t));
+		// The rows above and below, then the columns.
+		const int side = k - 2 * kHaloW;
+		const int tx = side < 0 ? (k < kHaloW ? k : k - kHaloW) : (side < kTileH ? 0 : kHaloW - 1);
+		const int ty = side < 0 ? (k < kHaloW ? 0 : kHaloH - 1) : (side < kTileH ? side : side - kTileH) + 1;
+		const int t = min(max(y0 + ty - 1, 0), H - 1) * W + min(max(x0 + tx - 1, 0), W - 1);
+		storeTexel(tile, tx, ty, compress(loadH3(hdr, t)), loadF1(depth, t));
 	}
 }
 
 // fs_taa.sc:111-172 for pixel (x, y), at (lx, ly) in the block's tile.
-__device__ __forceinline__ V4 taaPixel(const RestirDisplayParams& P, const uint16_t* __restrict__ hdr,
-	const float4* tile, const uint16_t* __restrict__ history, int x, int y, int lx, int ly)
+__device__ __forceinline__ V4 taaPixel(const RestirDisplayParams& P, V4 current, V3 compressed, const float4* tile,
+	const uint16_t* __restrict__ history, int x, int y, int lx, int ly)
 {
 	const int W = int(P.width), H = int(P.height);
 	const V2 texel = v2(1.0f / float(W), 1.0f / float(H));
 	const V2 uv = v2((float(x) + 0.5f) * texel.x, (float(y) + 0.5f) * texel.y);
-	const V4 current = loadH4(hdr, texelIndex(uv, W, H));
 
 	V3 sum = v3s(0.0f);
 	V3 sumSquares = v3s(0.0f);
@@ -205,7 +225,7 @@ __device__ __forceinline__ V4 taaPixel(const RestirDisplayParams& P, const uint1
 	const V3 deviation = v3(sqrtf(variance.x), sqrtf(variance.y), sqrtf(variance.z));
 	V3 past = toYCoCg(compress(sampleHistory(history, W, H, previousUv, texel)));
 	past = clipToBox(past, mean, deviation * 1.25f);
-	const V3 blended = mix(fromYCoCg(past), compress(current.xyz()), 0.1f);
+	const V3 blended = mix(fromYCoCg(past), compressed, 0.1f);
 	V3 result = decompress(blended);
 	if (anyNan(result))
 	{
@@ -248,19 +268,32 @@ __device__ __forceinline__ float agxLog(float v, float minEv, float maxEv)
 	return clampf(rn_log2(fmaxf(v, 1e-10f)), minEv, maxEv);
 }
 
-__device__ __forceinline__ V3 tonemapAgx(V3 c)
+// x / 16.5 (the stops from minEv to maxEv), rounded as the division: a product
+// with the reciprocal and one correction by its remainder, exact (Brisebarre,
+// Muller and Raina, "Accelerating correctly rounded floating-point division
+// when the divisor is known in advance"). Equal for every float from 4e-37
+// to 17; x is 0 or at least 4e-7 here.
+__device__ __forceinline__ float agxShare(float x)
+{
+	constexpr float kShare = 1.0f / 16.5f;
+	const float q = x * kShare;
+	return __fmaf_rn(__fmaf_rn(-q, 16.5f, x), kShare, q);
+}
+
+// AgX up to its final power.
+__device__ __forceinline__ V3 agxDisplay(V3 c)
 {
 	const float minEv = -12.47393f;
 	const float maxEv = 4.026069f;
 	V3 color = mulRows(0.842479062253094f, 0.0784335999999992f, 0.0792237451477643f, 0.0423282422610123f, 0.878468636469772f,
 		0.0791661274605434f, 0.0423756549057051f, 0.0784336f, 0.879142973793104f, vmax(c, v3s(0.0f)));
 	color = v3(agxLog(color.x, minEv, maxEv), agxLog(color.y, minEv, maxEv), agxLog(color.z, minEv, maxEv));
-	color = (color - minEv) / (maxEv - minEv);
+	const V3 ev = color - minEv;
+	color = v3(agxShare(ev.x), agxShare(ev.y), agxShare(ev.z));
 	color = agxContrast(color);
 	color = mulRows(1.19687900512017f, -0.0980208811401368f, -0.0990297440797205f, -0.0528968517574562f, 1.15190312990417f,
 		-0.0989611768448433f, -0.0529716355144438f, -0.0980434501171241f, 1.15107367264116f, color);
-	color = clamp01(color);
-	return v3(rn_pow(color.x, 2.2f), rn_pow(color.y, 2.2f), rn_pow(color.z, 2.2f));
+	return clamp01(color);
 }
 
 __device__ __forceinline__ V3 tonemapNeutral(V3 c)
@@ -282,6 +315,7 @@ __device__ __forceinline__ V3 tonemapNeutral(V3 c)
 	return clamp01(mix(color, v3s(newPeak), g));
 }
 
+// The operator's colour; AgX's before its power of 2.2.
 __device__ __forceinline__ V3 tonemap(V3 c, int op)
 {
 	if (op == RESTIR_TONEMAP_ACES)
@@ -290,7 +324,7 @@ __device__ __forceinline__ V3 tonemap(V3 c, int op)
 	}
 	if (op == RESTIR_TONEMAP_AGX)
 	{
-		return tonemapAgx(c);
+		return agxDisplay(c);
 	}
 	if (op == RESTIR_TONEMAP_NEUTRAL)
 	{
@@ -323,9 +357,49 @@ __device__ __forceinline__ V4 background()
 	return v4(0.125f, 0.141f, 0.169f, 1.0f);
 }
 
+// A channel of the display: rn_unorm8(rn_pow(color, 1 / 2.2)), color itself
+// raised to 2.2 first when agx.
+__device__ __noinline__ uint32_t gammaByteExact(float color, bool agx)
+{
+	return rn_unorm8(rn_pow(fabsf(agx ? rn_pow(color, 2.2f) : color), 1.0f / 2.2f));
+}
+
+// The same, from an approximation where its rounding cannot be wrong: the
+// powers were a quarter of the pixel's instructions. AgX's two powers undo
+// each other, so color itself is the approximation; the other operators take
+// __powf. For every float of [0, 1] (of [0, inf] with __powf) the bytes differ
+// within 3.1e-5 of the edge between two bytes, if at all, and only there the
+// powers decide, as for NaN. (kGammaEdge 1e-3 sent 6 pixels of 1,000 and so a
+// sixth of the warps to them: 0.384 ms where 1e-4 took 0.335, all powers 0.423.)
+constexpr float kGammaEdge = 1e-4f;
+
+__device__ __forceinline__ uint32_t gammaByte(float color, bool agx)
+{
+	const float value = agx ? color : __powf(fabsf(color), 1.0f / 2.2f);
+	const float t = (value > 1.0f ? 1.0f : value) * 255.0f + 0.5f;
+	const float part = t - floorf(t);
+	return part > kGammaEdge && part < 1.0f - kGammaEdge ? uint32_t(t) : gammaByteExact(color, agx);
+}
+
+__device__ __forceinline__ void storeBytes(uint8_t* p, size_t i, uint32_t r, uint32_t g, uint32_t b)
+{
+	reinterpret_cast<uint32_t*>(p)[i] = b | (g << 8) | (r << 16) | 0xff000000u;
+}
+
+// The factor on the image's radiance (fs_tonemap.sc:106-118).
+__device__ __forceinline__ float exposureScale(const RestirDisplayParams& P, const uint32_t* __restrict__ exposure)
+{
+	float scale = rn_exp2(P.exposure_ev);
+	if (P.auto_exposure > 0.5f && P.pass_through <= 0.5f)
+	{
+		scale = scale * (0.18f / rn_exp2(__uint_as_float(*exposure)));
+	}
+	return scale;
+}
+
 // fs_tonemap.sc:122-162 for pixel i.
-__device__ __forceinline__ V4 tonemapPixel(const RestirDisplayParams& P, V4 hdr, const uint32_t* __restrict__ exposure,
-	const double* __restrict__ mean, const uint8_t* __restrict__ alpha, size_t i, size_t n)
+__device__ __forceinline__ void tonemapPixel(const RestirDisplayParams& P, V4 hdr, float scale,
+	const double* __restrict__ mean, const uint8_t* __restrict__ alpha, size_t i, size_t n, uint8_t* __restrict__ display)
 {
 	if (P.reference_view > 1.5f)
 	{
@@ -334,28 +408,22 @@ __device__ __forceinline__ V4 tonemapPixel(const RestirDisplayParams& P, V4 hdr,
 		const float imageLuminance = luminance(hdr.xyz());
 		const float referenceLuminance = luminance(reference);
 		const float error = (imageLuminance - referenceLuminance) / fmaxf(referenceLuminance, 0.01f);
-		return referenceAlpha < 0.5f ? background() : v4(turbo(0.5f + clampf(error, -0.5f, 0.5f)), 1.0f);
+		storeU8(display, int(i), referenceAlpha < 0.5f ? background() : v4(turbo(0.5f + clampf(error, -0.5f, 0.5f)), 1.0f));
+		return;
 	}
 	if (P.reference_view > 0.5f)
 	{
 		hdr = v4(float(mean[i]), float(mean[n + i]), float(mean[2 * n + i]), alpha[i] ? 1.0f : 0.0f);
 	}
-	if (P.pass_through > 0.5f)
+	if (P.pass_through > 0.5f || hdr.w < 0.5f)
 	{
-		return v4(hdr.xyz(), 1.0f);
+		storeU8(display, int(i), P.pass_through > 0.5f ? v4(hdr.xyz(), 1.0f) : background());
+		return;
 	}
-	if (hdr.w < 0.5f)
-	{
-		return background();
-	}
-	float scale = rn_exp2(P.exposure_ev);
-	if (P.auto_exposure > 0.5f)
-	{
-		scale = scale * (0.18f / rn_exp2(__uint_as_float(*exposure)));
-	}
-	const V3 color = tonemap(hdr.xyz() * scale, int(P.tonemapper));
-	const float gamma = 1.0f / 2.2f;
-	return v4(rn_pow(fabsf(color.x), gamma), rn_pow(fabsf(color.y), gamma), rn_pow(fabsf(color.z), gamma), 1.0f);
+	const int op = int(P.tonemapper);
+	const V3 color = tonemap(hdr.xyz() * scale, op);
+	const bool agx = op == RESTIR_TONEMAP_AGX;
+	storeBytes(display, i, gammaByte(color.x, agx), gammaByte(color.y, agx), gammaByte(color.z, agx));
 }
 
 // A value as the RGBA16F target holds it.
@@ -366,21 +434,33 @@ __device__ __forceinline__ V4 roundHalf4(V4 v)
 }
 
 template<int kMode>
-__global__ void __launch_bounds__(128, RESTIR_DISPLAY_MIN_BLOCKS) displayKernel(const RestirDisplayParams P, const uint16_t* __restrict__ hdr,
+__global__ void __launch_bounds__(kTileW * kTileH, RESTIR_DISPLAY_MIN_BLOCKS) displayKernel(const RestirDisplayParams P, const uint16_t* __restrict__ hdr,
 	const float* __restrict__ depth, const uint16_t* __restrict__ history, uint16_t* __restrict__ taaOut,
 	const uint32_t* __restrict__ exposure, const double* __restrict__ mean, const uint8_t* __restrict__ alpha,
 	uint8_t* __restrict__ display)
 {
 	__shared__ float4 tile[kHaloW * kHaloH];
+	__shared__ float sharedScale;
 	const int W = int(P.width), H = int(P.height);
+	if ((kMode & kModeTonemap) && threadIdx.x >= 96u)
+	{
+		// One warp for the block: the two powers are 4% of a pixel's instructions.
+		const float scale = exposureScale(P, exposure);
+		if (threadIdx.x == 96u)
+		{
+			sharedScale = scale;
+		}
+	}
 	const int lx = int(threadIdx.x) % kTileW, ly = int(threadIdx.x) / kTileW;
 	const int x = int(blockIdx.x) * kTileW + lx;
 	const int y = int(blockIdx.y) * kTileH + ly;
+	V4 current;
+	V3 compressed;
 	if (kMode & kModeTaa)
 	{
-		loadNeighbourhood(tile, hdr, depth, W, H, int(blockIdx.x) * kTileW, int(blockIdx.y) * kTileH);
-		__syncthreads();
+		loadNeighbourhood(tile, hdr, depth, W, H, int(blockIdx.x) * kTileW, int(blockIdx.y) * kTileH, lx, ly, current, compressed);
 	}
+	__syncthreads();
 	if (x >= W || y >= H)
 	{
 		return;
@@ -389,7 +469,7 @@ __global__ void __launch_bounds__(128, RESTIR_DISPLAY_MIN_BLOCKS) displayKernel(
 	V4 color;
 	if (kMode & kModeTaa)
 	{
-		color = taaPixel(P, hdr, tile, history, x, y, lx, ly);
+		color = taaPixel(P, current, compressed, tile, history, x, y, lx, ly);
 		storeH4(taaOut, i, color);
 		color = roundHalf4(color);
 	}
@@ -399,7 +479,7 @@ __global__ void __launch_bounds__(128, RESTIR_DISPLAY_MIN_BLOCKS) displayKernel(
 	}
 	if (kMode & kModeTonemap)
 	{
-		storeU8(display, i, tonemapPixel(P, color, exposure, mean, alpha, size_t(i), size_t(W) * size_t(H)));
+		tonemapPixel(P, color, sharedScale, mean, alpha, size_t(i), size_t(W) * size_t(H), display);
 	}
 }
 

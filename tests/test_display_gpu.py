@@ -181,3 +181,43 @@ def test_renderer_display_chain_equals_pass_by_pass_frames():
     np.testing.assert_array_equal(renderer.download("display.hdr", np.uint16)[:w * h * 4],
                                   runner.host(runner.displayed()))
     np.testing.assert_array_equal(renderer.download("exposure", np.uint32)[:1], runner.host("exposure"))
+
+
+@pytest.mark.parametrize("tonemapper", range(5))
+def test_tonemap_bytes_at_their_edges(tonemapper):
+    """Values on both sides of every edge between two bytes, and a dense sweep of
+    greys and colours: the bytes are the powers', whichever way they were found."""
+    w, h = 640, 400
+    rng = np.random.default_rng(5)
+    edge = (((np.arange(1, 256) - 0.5) / 255.0) ** 2.2).astype(np.float32).view(np.int32)
+    edges = (edge[:, None] + np.arange(-40, 41)[None, :]).astype(np.int32).view(np.float32).reshape(-1)
+    sweep = np.exp(np.linspace(np.log(1e-5), np.log(40.0), w * h - edges.size))
+    grey = np.concatenate([edges.astype(np.float64), sweep])
+    mean = np.stack([grey, grey * np.where(rng.random(w * h) < 0.5, 1.0, rng.random(w * h)), grey[::-1]])
+    alpha = np.ones(w * h, np.uint8)
+    inputs = display_inputs(w, h, seed=3)
+    p = display_params(w, h, inputs, tonemapper=float(tonemapper), exposure_ev=0.0, auto_exposure=0.0, reference_view=1.0)
+    expected = np.zeros(w * h * 4, np.uint8)
+    ob.load().oracle_tonemap(C.byref(p), inputs["hdr"].ctypes.data, None, mean.ctypes.data, alpha.ctypes.data,
+                             expected.ctypes.data)
+    hdr, mean_d, alpha_d = device(inputs["hdr"]), device(mean), device(alpha)
+    out = device(np.zeros(w * h * 4, np.uint8))
+    rb.check(rb.load().restir_tonemap(C.byref(p), hdr.data_ptr(), None, mean_d.data_ptr(), alpha_d.data_ptr(),
+                                      out.data_ptr(), None), "restir_tonemap")
+    np.testing.assert_array_equal(host(out), expected)
+
+
+@pytest.mark.parametrize("size", [(1, 1), (31, 17), (33, 15), (32, 16), (65, 33)])
+def test_display_tile_edges(size):
+    """Images of a part of a tile, of whole tiles and of one pixel more."""
+    w, h = size
+    inputs = display_inputs(w, h, seed=40 + w)
+    p = display_params(w, h, inputs, taa=1.0, taa_history_valid=1.0)
+    expected = np.zeros_like(inputs["hdr"])
+    ob.load().oracle_taa(C.byref(p), inputs["hdr"].ctypes.data, inputs["depth"].ctypes.data,
+                         inputs["history"].ctypes.data, expected.ctypes.data)
+    hdr, depth, history = device(inputs["hdr"]), device(inputs["depth"]), device(inputs["history"])
+    out = device(np.zeros_like(inputs["hdr"]))
+    rb.check(rb.load().restir_taa(C.byref(p), hdr.data_ptr(), depth.data_ptr(), history.data_ptr(), out.data_ptr(), None),
+             "restir_taa")
+    np.testing.assert_array_equal(host(out), expected)
