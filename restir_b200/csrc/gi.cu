@@ -369,51 +369,108 @@ __global__ void __launch_bounds__(128, RESTIR_GI_SPATIAL_MIN_BLOCKS) giSpatialKe
 
 	const float radius = g.reuseRadius(position);
 	PairwiseMis mis = g.beginPairwiseMis(position, normal, canonical, canonicalCount, P.spatial_taps);
-	for (int tapIndex = 0; tapIndex < P.spatial_taps; ++tapIndex)
+	// The taps and the combination (the last step) as one loop with one call site
+	// of the visibility test, in three parts with a barrier before each. The
+	// kernel is bound by instruction fetch and divergence: the barriers bring a
+	// warp's lanes together again before the test and the evaluation, and keep
+	// a block's warps in the same part of the code, so that they fetch it once.
+	// (Pixels without a surface have left; a barrier counts the others.) 0.942 ms
+	// for the 960x540 pixels of the 1M-triangle city, 0.578 for the
+	// 100k-triangle courtyard's 640x360, 0.205 for 256x256 in the Cornell box;
+	// without barriers 1.197, 0.794, 0.219, with a warp's barriers only 1.034,
+	// 0.621, 0.201, as a plain loop of neighbours 1.197, 0.720, 0.204. Blocks of
+	// 64 and 256 threads: 1.005 and 0.989 ms in the city.
+	float combinedWeight = 0.0f;
+	const int taps = max(P.spatial_taps, 0);
+#pragma unroll 1
+	for (int tapIndex = 0; tapIndex <= taps; ++tapIndex)
 	{
-		float random0 = nextRandom(rng);
-		float random1 = nextRandom(rng);
-		float random2 = nextRandom(rng);
-		float randomSelect = nextRandom(rng);
-		V2 neighbourUv = v2(-1.0f, -1.0f);
-		if (g.grid.worldSpace)
+		__syncthreads();
+		NeighbourReservoir neighbour;
+		float neighbourGeometry = 0.0f;
+		float randomSelect = 0.0f;
+		bool accepted = false;
+		bool test = false;
+		V3 from = position, fromNormal = normal, to = v3s(0.0f);
+		float toId = 0.0f;
+		if (tapIndex < taps)
 		{
-			uint32_t entry = gridPickEntry(g.grid, position, normal, random0, random1, random2);
-			if (entry != kGridInvalid && entry != pixelIndex)
+			float random0 = nextRandom(rng);
+			float random1 = nextRandom(rng);
+			float random2 = nextRandom(rng);
+			randomSelect = nextRandom(rng);
+			V2 neighbourUv = v2(-1.0f, -1.0f);
+			if (g.grid.worldSpace)
 			{
-				neighbourUv = g.giPixelUv(entry);
+				uint32_t entry = gridPickEntry(g.grid, position, normal, random0, random1, random2);
+				if (entry != kGridInvalid && entry != pixelIndex)
+				{
+					neighbourUv = g.giPixelUv(entry);
+				}
+			}
+			else
+			{
+				float diskRadius = 12.0f * sqrtf(random0);
+				float angle = 2.0f * kPi * random1;
+				float sn, cs;
+				rn_sincos(angle, &sn, &cs);
+				V2 neighbourPixel = v2(floorf(pixel.x + cs * diskRadius), floorf(pixel.y + sn * diskRadius));
+				if (neighbourPixel.x != pixel.x || neighbourPixel.y != pixel.y)
+				{
+					neighbourUv = v2((neighbourPixel.x + 0.5f) * g.giTexel.x, (neighbourPixel.y + 0.5f) * g.giTexel.y);
+				}
+			}
+			if (isOnScreen(neighbourUv))
+			{
+				int i = g.gi(neighbourUv);
+				accepted = g.acceptNeighbour(f4(b.reservoirSample[i]), f4(b.reservoirReceiver[i]), f4(b.reservoirNormal[i]),
+					position, normal, radius, neighbour);
+				neighbour.cacheSlot = g.cache != nullptr ? g.cacheNeighbourBase + i : -1;
+			}
+			if (!accepted)
+			{
+				GiPass::skipNeighbour(mis);
+			}
+			else
+			{
+				test = g.neighbourBegin(mis, neighbour, neighbourGeometry);
+				from = neighbour.receiverPosition;
+				fromNormal = neighbour.receiverNormal;
+				to = mis.canonicalPosition;
+				toId = mis.canonicalId;
 			}
 		}
 		else
 		{
-			float diskRadius = 12.0f * sqrtf(random0);
-			float angle = 2.0f * kPi * random1;
-			float sn, cs;
-			rn_sincos(angle, &sn, &cs);
-			V2 neighbourPixel = v2(floorf(pixel.x + cs * diskRadius), floorf(pixel.y + sn * diskRadius));
-			if (neighbourPixel.x != pixel.x || neighbourPixel.y != pixel.y)
+			test = g.finishBegin(mis, canonical, canonicalWeight, nextRandom(rng), combinedWeight);
+			to = mis.combined.position;
+			toId = mis.combined.id;
+		}
+		__syncthreads();
+		const bool occluded = test && !g.template isVisible<kWave>(from, fromNormal, to, toId);
+		if (tapIndex == taps)
+		{
+			if (occluded)
 			{
-				neighbourUv = v2((neighbourPixel.x + 0.5f) * g.giTexel.x, (neighbourPixel.y + 0.5f) * g.giTexel.y);
+				combinedWeight = 0.0f;
 			}
+			break;
 		}
-		NeighbourReservoir neighbour;
-		bool accepted = false;
-		if (isOnScreen(neighbourUv))
+		__syncthreads();
+		if (accepted)
 		{
-			int i = g.gi(neighbourUv);
-			accepted = g.acceptNeighbour(f4(b.reservoirSample[i]), f4(b.reservoirReceiver[i]), f4(b.reservoirNormal[i]),
-				position, normal, radius, neighbour);
-			neighbour.cacheSlot = g.cache != nullptr ? g.cacheNeighbourBase + i : -1;
+			g.neighbourShare(mis, neighbour, neighbourGeometry, occluded);
+			V3 contribution = v3s(0.0f);
+			V3 sampleNormal = v3(0.0f, 0.0f, 1.0f);
+			bool shifted = false;
+			if (neighbour.weight > 0.0f)
+			{
+				shifted = g.evaluateSample(position, normal, albedo, neighbour.samplePosition, neighbour.sampleId, contribution,
+					sampleNormal, neighbour.cacheSlot);
+			}
+			g.neighbourShift(mis, position, normal, neighbour, shifted, contribution, sampleNormal, randomSelect);
 		}
-		if (!accepted)
-		{
-			GiPass::skipNeighbour(mis);
-			continue;
-		}
-		g.template addNeighbour<kWave>(mis, position, normal, albedo, neighbour, randomSelect);
 	}
-
-	const float combinedWeight = g.template finishPairwiseMis<kWave>(mis, position, normal, canonical, canonicalWeight, nextRandom(rng));
 	V3 estimate = mis.combined.contribution * combinedWeight;
 	if (P.outlier_clamp > 0.0f)
 	{
@@ -602,7 +659,10 @@ __global__ void __launch_bounds__(kGiThreads, RESTIR_GI_TEMPORAL_MIN_BLOCKS) giT
 	// fetch): steps 0..C-1 shade the candidates, steps C..C+T-1 take the
 	// temporal neighbours and step C+T combines, the last two for working
 	// pixels only. The random draws and every operation are the
-	// straight-line form's, in its order.
+	// straight-line form's, in its order. Each step has three parts with a
+	// barrier before each, as in giSpatialKernel: 0.638 ms (960x540, city),
+	// 0.380 (640x360, courtyard), 0.132 (256x256, Cornell box); as one part,
+	// left early by lanes without a neighbour, 0.767, 0.457, 0.146.
 	const int candidates = P.initial_candidates;
 	const int taps = P.temporal_taps;
 	const int last = working ? candidates + taps : candidates - 1;
@@ -620,9 +680,11 @@ __global__ void __launch_bounds__(kGiThreads, RESTIR_GI_TEMPORAL_MIN_BLOCKS) giT
 	float combinedWeight = 0.0f;
 	bool misStarted = false;
 #pragma unroll 1
-	for (int step = 0; step <= last; ++step)
+	for (int step = 0; step <= candidates + taps; ++step)
 	{
-		if (step >= candidates && !misStarted)
+		__syncthreads();
+		bool active = step <= last;
+		if (active && step >= candidates && !misStarted)
 		{
 			canonicalWeight = canonical.target > 0.000001f ? canonical.weightSum / (canonical.count * canonical.target) : 0.0f;
 			mis = g.beginPairwiseMis(position, normal, canonical, canonical.count, taps);
@@ -640,7 +702,7 @@ __global__ void __launch_bounds__(kGiThreads, RESTIR_GI_TEMPORAL_MIN_BLOCKS) giT
 		bool test = false;
 		V3 from = position, fromNormal = normal, to = v3s(0.0f);
 		float toId = 0.0f;
-		if (step < candidates)
+		if (step < candidates && active)
 		{
 			const int sampleIndex = step;
 			float random0 = nextRandom(rng);
@@ -683,7 +745,7 @@ __global__ void __launch_bounds__(kGiThreads, RESTIR_GI_TEMPORAL_MIN_BLOCKS) giT
 			evaluate = hit;
 			cacheSlot = g.cache != nullptr ? pixel * records.candidates + sampleIndex : -1;
 		}
-		else if (step < candidates + taps)
+		else if (step < candidates + taps && active)
 		{
 			const int tapIndex = step - candidates;
 			float random0 = nextRandom(rng);
@@ -717,20 +779,24 @@ __global__ void __launch_bounds__(kGiThreads, RESTIR_GI_TEMPORAL_MIN_BLOCKS) giT
 			if (!accepted)
 			{
 				GiPass::skipNeighbour(mis);
-				continue;
+				active = false;
 			}
-			test = g.neighbourBegin(mis, neighbour, neighbourGeometry);
-			from = neighbour.receiverPosition;
-			fromNormal = neighbour.receiverNormal;
-			to = mis.canonicalPosition;
-			toId = mis.canonicalId;
+			else
+			{
+				test = g.neighbourBegin(mis, neighbour, neighbourGeometry);
+				from = neighbour.receiverPosition;
+				fromNormal = neighbour.receiverNormal;
+				to = mis.canonicalPosition;
+				toId = mis.canonicalId;
+			}
 		}
-		else
+		else if (active)
 		{
 			test = g.finishBegin(mis, canonical, canonicalWeight, nextRandom(rng), combinedWeight);
 			to = mis.combined.position;
 			toId = mis.combined.id;
 		}
+		__syncthreads();
 		const bool occluded = test && !g.template isVisible<kWave>(from, fromNormal, to, toId);
 		if (step == candidates + taps)
 		{
@@ -739,6 +805,11 @@ __global__ void __launch_bounds__(kGiThreads, RESTIR_GI_TEMPORAL_MIN_BLOCKS) giT
 				combinedWeight = 0.0f;
 			}
 			break;
+		}
+		__syncthreads();
+		if (!active)
+		{
+			continue;
 		}
 		if (step >= candidates)
 		{
