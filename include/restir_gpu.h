@@ -431,6 +431,12 @@ int restir_counters(int enable, uint64_t* counters);
  * counterpart in the reference (a test hook). */
 int restir_numeric_eval(int fn, const float* input, float* output, uint32_t n, void* stream);
 
+/* Which of a pass's two instances the traversal of a scene takes (a check for
+ * tests, no counterpart in the reference): 1 when its BVH rows are read 32
+ * bytes at a time (bvh starts on 32 bytes and triangle_offset is even), 0 when
+ * 16 at a time. Looks at the struct only. */
+int restir_bvh_wide_rows(const RestirScene* scene);
+
 /* A bandwidth probe with the traversal kernels' fetch pattern (a measurement
  * hook, no counterpart in the reference): blocks x 256 threads each gather
  * `gathers` rows of 32 bytes (two 16-byte read-only loads, the size of a BVH

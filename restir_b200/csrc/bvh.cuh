@@ -466,10 +466,13 @@ __device__ __forceinline__ float slabEnter(const SlabRay& r, const NodeRow& n, f
 	return enter <= leave ? enter : -1.0f;
 }
 
-// Whether a scene's nodes can be read 32 bytes at a time.
+// Whether a scene's nodes (two rows each) and the first two rows of its
+// triangles (four rows each, from triangleOffset on) can be read 32 bytes at a
+// time: both start on 32 bytes when the buffer does and the offset is even. The
+// offset is the caller's, and any padding may lie before the triangles.
 __host__ inline bool wideRows(const BvhView& b)
 {
-	return (reinterpret_cast<uintptr_t>(b.rows) & 31u) == 0u;
+	return (reinterpret_cast<uintptr_t>(b.rows) & 31u) == 0u && (b.triangleOffset & 1) == 0;
 }
 
 // Nearest hit in (0, distance) among the triangles accept() lets through,

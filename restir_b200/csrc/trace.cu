@@ -195,6 +195,11 @@ void launchParts(const BvhView& bvh, const RayArrays& arrays, uint32_t n, int ki
 
 using namespace restir;
 
+extern "C" int restir_bvh_wide_rows(const RestirScene* scene)
+{
+	return scene != nullptr && wideRows(makeBvhView(scene)) ? 1 : 0;
+}
+
 extern "C" int restir_trace(const RestirParams* params, const RestirScene* scene, const float* rays,
 	int32_t* hit_triangle, float* hit_distance, uint32_t n, int kind, void* stream)
 {

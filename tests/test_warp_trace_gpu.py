@@ -8,6 +8,7 @@ import pytest
 
 import oracle.binding as ob
 import restir_b200 as rb
+from restir_b200.abi import RestirScene
 from tests.helpers import SceneSetup, make_scene, seeded_rays
 
 KINDS = [rb.TRACE_CLOSEST, rb.TRACE_ANY, rb.TRACE_CLOSEST_STACKLESS, rb.TRACE_CLOSEST_QUEUE]
@@ -93,3 +94,30 @@ def test_unaligned_rows(kind):
     """16 bytes past a 32-byte boundary: the nodes are read with 128-bit loads."""
     setup = make_scene(rb.SCENE_CITY, 0, 60_000)
     check(setup, seeded_rays(setup, 20_000, seed=8), kind, offset=4)
+
+
+def test_wide_rows_rule():
+    """32-byte reads need the nodes and the triangles on 32 bytes: a buffer on 16 bytes only, or an odd number of rows
+    before the triangles, takes the 16-byte ones."""
+    scene = RestirScene()
+    for address, offset, wide in ((4096, 86, 1), (4096, 87, 0), (4112, 86, 0), (4112, 87, 0), (4128, 0, 1)):
+        scene.bvh, scene.node_count, scene.triangle_offset, scene.triangle_count = address, 43, offset, 36
+        assert rb.load().restir_bvh_wide_rows(scene) == wide, (address, offset)
+    assert rb.load().restir_bvh_wide_rows(None) == 0
+
+
+def padded(setup: SceneSetup, rows: int) -> SceneSetup:
+    """setup with rows of padding between its nodes and its triangles."""
+    data, offset = setup.bvh.data.reshape(-1, 4), setup.bvh.desc.triangle_offset
+    setup.bvh_data = np.concatenate([data[:offset], np.full((rows, 4), np.nan, np.float32), data[offset:]]).reshape(-1)
+    setup.node_count, setup.triangle_offset = setup.bvh.desc.node_count, offset + rows
+    return setup
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", KINDS + [rb.TRACE_CLOSEST_WATERTIGHT, rb.TRACE_ANY_WAVE])
+@pytest.mark.parametrize("rows", [1, 2, 3])
+def test_padding_before_the_triangles(kind, rows):
+    """Triangles that start on 16 bytes only, and on 32 again."""
+    setup = padded(make_scene(rb.SCENE_CITY, 0, 60_000), rows)
+    check(setup, seeded_rays(setup, 20_000, seed=9), kind)
