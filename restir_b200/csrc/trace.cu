@@ -51,7 +51,7 @@ struct PartSource
 		const uint32_t rank = uint32_t(idleRank<kLanes>(mask));
 		if (idle && rank < left)
 		{
-			arrays.load(int(next + rank), r);
+			arrays.load(next + rank, r);
 		}
 		next += min(wanted, left);
 		more = left > wanted;
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(kTraceBlock) traceKernel(BvhView bvh, RayArray
 		return;
 	}
 	Ray r;
-	arrays.load(int(i), r);
+	arrays.load(i, r);
 	const float length = r.distance;
 	if (kKind == RESTIR_TRACE_CLOSEST)
 	{
@@ -140,7 +140,8 @@ __global__ void __launch_bounds__(kTraceBlock) traceKernel(BvhView bvh, RayArray
 template<int kKind, bool kWide = false>
 void launchThreads(const BvhView& bvh, const RayArrays& arrays, uint32_t n, cudaStream_t s)
 {
-	traceKernel<kKind, kWide><<<(n + kTraceBlock - 1) / kTraceBlock, kTraceBlock, 0, s>>>(bvh, arrays, n);
+	const uint32_t blocks = uint32_t((uint64_t(n) + kTraceBlock - 1) / kTraceBlock);
+	traceKernel<kKind, kWide><<<blocks, kTraceBlock, 0, s>>>(bvh, arrays, n);
 }
 
 // Rays per warp: as few as fill the SMs once (148 x 32 warps resident), a

@@ -134,17 +134,20 @@ __device__ __forceinline__ bool testLeaves(const BvhView& b, LeafSlots& slots, b
 // traceNearest, traceLaneWalks and traceGroupWalks trace rays until their source has no more. Every
 // lane of the warp calls them. A source gives
 //   take(idle, more, r): called by the whole warp; an idle lane (traceGroupWalks:
-//     the four lanes of an idle group) gets a ray in r, r.index -1 when there is
-//     none for it, and more is cleared when there are none left;
+//     the four lanes of an idle group) gets a ray in r, r.index stays kNoRay when
+//     there is none for it, and more is cleared when there are none left;
 //   store(r): the ray's hit and distance;
 //   kCount: the kind of ray to count (-1: a ray counted before).
+
+// A ray set has up to 2^32 - 1 rays (restir_trace's n), the last index is free.
+constexpr uint32_t kNoRay = 0xffffffffu;
 
 struct Ray
 {
 	V3 o, d;
 	float distance;  // the nearest hit's, or the ray's length
 	int hit;
-	int index;       // -1: none
+	uint32_t index;  // kNoRay: none
 };
 
 // The lanes' takers: one per lane (kLanes 1) or one per group of kLanes lanes,
@@ -207,7 +210,7 @@ __device__ __forceinline__ void traceNearest(const BvhView& b, Source& source, N
 	constexpr int kStep = 0, kLeaf = 1, kDone = 2;
 	int mode = kDone;
 	Ray r = {};
-	r.index = -1;
+	r.index = kNoRay;
 	SlabRay slab = {};
 	// The node to visit: (node, -a) of an interior node or (a's bits, b) of a
 	// leaf, told apart by the second word's sign, so that a child's words, read
@@ -286,22 +289,22 @@ __device__ __forceinline__ void traceNearest(const BvhView& b, Source& source, N
 	for (;;)
 	{
 		// Rays that have ended are stored, and lanes without one take the next.
-		const unsigned done = __ballot_sync(kAll, mode == kDone && (r.index >= 0 || more));
+		const unsigned done = __ballot_sync(kAll, mode == kDone && (r.index != kNoRay || more));
 		if (__popc(done) >= RESTIR_TRACE_REFILL || (done != 0u && __all_sync(kAll, mode == kDone)))
 		{
-			if (mode == kDone && r.index >= 0)
+			if (mode == kDone && r.index != kNoRay)
 			{
 				// The root, and both children of each interior node visited.
 				countWork(Source::kCount, 1u + 2u * uint32_t(step - leafVisits), triangles);
 				r.hit = dropped ? markedHit(r.hit) : r.hit;
 				source.store(r);
-				r.index = -1;
+				r.index = kNoRay;
 			}
 			if (more)
 			{
-				const bool idle = r.index < 0;
+				const bool idle = r.index == kNoRay;
 				source.take(idle, more, r);
-				if (idle && r.index >= 0)
+				if (idle && r.index != kNoRay)
 				{
 					slab = slabRay(r.o, r.d);
 					step = 0;
@@ -323,7 +326,7 @@ __device__ __forceinline__ void traceNearest(const BvhView& b, Source& source, N
 				}
 			}
 		}
-		const int active = __popc(__ballot_sync(kAll, r.index >= 0));
+		const int active = __popc(__ballot_sync(kAll, r.index != kNoRay));
 		if (active == 0 && !more)
 		{
 			break;
@@ -373,7 +376,7 @@ __device__ __forceinline__ void traceGroupWalks(const BvhView& b, Source& source
 	constexpr unsigned kAll = 0xffffffffu;
 	constexpr int kAtLeaf = 0x7fffffff;
 	Ray r = {};
-	r.index = -1;
+	r.index = kNoRay;
 	SlabRay slab = {};
 	int node = 0;           // the walk's next node
 	int step = 0;
@@ -386,22 +389,22 @@ __device__ __forceinline__ void traceGroupWalks(const BvhView& b, Source& source
 	for (;;)
 	{
 		// Rays that have ended are stored, and groups without one take the next.
-		if (__any_sync(kAll, !go && !waiting && (r.index >= 0 || more)))
+		if (__any_sync(kAll, !go && !waiting && (r.index != kNoRay || more)))
 		{
-			if (!go && !waiting && r.index >= 0)
+			if (!go && !waiting && r.index != kNoRay)
 			{
 				if (sub == 0)
 				{
 					countWork(Source::kCount, uint32_t(step), triangles);
 					source.store(r);
 				}
-				r.index = -1;
+				r.index = kNoRay;
 			}
 			if (more)
 			{
-				const bool take = r.index < 0;
+				const bool take = r.index == kNoRay;
 				source.take(take, more, r);
-				if (take && r.index >= 0)
+				if (take && r.index != kNoRay)
 				{
 					slab = slabRay(r.o, r.d);
 					node = 0;
@@ -411,7 +414,7 @@ __device__ __forceinline__ void traceGroupWalks(const BvhView& b, Source& source
 				}
 			}
 		}
-		const int rays = __popc(__ballot_sync(kAll, r.index >= 0));
+		const int rays = __popc(__ballot_sync(kAll, r.index != kNoRay));
 		if (rays == 0)
 		{
 			if (!more)
@@ -511,7 +514,7 @@ __device__ __forceinline__ void traceLaneWalks(const BvhView& b, Source& source,
 {
 	constexpr unsigned kAll = 0xffffffffu;
 	Ray r = {};
-	r.index = -1;
+	r.index = kNoRay;
 	SlabRay slab = {};
 	int node = 0;
 	int step = 0;
@@ -522,9 +525,9 @@ __device__ __forceinline__ void traceLaneWalks(const BvhView& b, Source& source,
 	bool more = true;
 	for (;;)
 	{
-		if (__any_sync(kAll, !go && !waiting && (r.index >= 0 || more)))
+		if (__any_sync(kAll, !go && !waiting && (r.index != kNoRay || more)))
 		{
-			if (!go && !waiting && r.index >= 0)
+			if (!go && !waiting && r.index != kNoRay)
 			{
 				if (step >= kBvhMaxSteps && !(kAny && r.hit >= 0))
 				{
@@ -532,13 +535,13 @@ __device__ __forceinline__ void traceLaneWalks(const BvhView& b, Source& source,
 				}
 				countWork(Source::kCount, uint32_t(step), triangles);
 				source.store(r);
-				r.index = -1;
+				r.index = kNoRay;
 			}
 			if (more)
 			{
-				const bool take = r.index < 0;
+				const bool take = r.index == kNoRay;
 				source.take(take, more, r);
-				if (take && r.index >= 0)
+				if (take && r.index != kNoRay)
 				{
 					slab = slabRay(r.o, r.d);
 					node = 0;
@@ -548,7 +551,7 @@ __device__ __forceinline__ void traceLaneWalks(const BvhView& b, Source& source,
 				}
 			}
 		}
-		const int rays = __popc(__ballot_sync(kAll, r.index >= 0));
+		const int rays = __popc(__ballot_sync(kAll, r.index != kNoRay));
 		if (rays == 0)
 		{
 			if (!more)

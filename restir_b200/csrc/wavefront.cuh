@@ -66,7 +66,7 @@ struct RayArrays
 	int* hitTriangle;
 	float* hitDistance;
 
-	__device__ __forceinline__ void load(int i, Ray& r) const
+	__device__ __forceinline__ void load(uint32_t i, Ray& r) const
 	{
 		const float4 a = rays[2 * size_t(i)];
 		const float4 c = rays[2 * size_t(i) + 1];
@@ -110,7 +110,7 @@ struct QueueSource
 		const uint32_t mine = start + uint32_t(idleRank<kLanes>(mask));
 		if (idle && mine >= start && mine < total)
 		{
-			arrays.load(int(mine), r);
+			arrays.load(mine, r);
 		}
 	}
 	__device__ __forceinline__ void store(const Ray& r) const { arrays.store(r); }
@@ -151,15 +151,15 @@ struct MarkedSource
 					more = false;
 					break;
 				}
-				next = base + 32u;
+				next = end - base > 32u ? base + 32u : end;
 				const uint32_t i = base + lane;
-				pending = __ballot_sync(0xffffffffu, i >= base && i < end && arrays.hitTriangle[i] < -1);
+				pending = __ballot_sync(0xffffffffu, lane < end - base && arrays.hitTriangle[i] < -1);
 				continue;
 			}
 			// The first idle group takes the first marked ray.
 			if ((lane & ~unsigned(kLanes - 1)) == unsigned(__ffs(mask) - 1))
 			{
-				const int i = int(base) + __ffs(pending) - 1;
+				const uint32_t i = base + uint32_t(__ffs(pending) - 1);
 				arrays.load(i, r);
 				r.hit = markedHit(arrays.hitTriangle[i]);
 				r.distance = arrays.hitDistance[i];

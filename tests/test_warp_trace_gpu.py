@@ -121,3 +121,35 @@ def test_padding_before_the_triangles(kind, rows):
     """Triangles that start on 16 bytes only, and on 32 again."""
     setup = padded(make_scene(rb.SCENE_CITY, 0, 60_000), rows)
     check(setup, seeded_rays(setup, 20_000, seed=9), kind)
+
+
+@pytest.mark.gpu
+def test_more_than_2_31_rays():
+    """Indices past 2^31: a set of rays that end before they start, and at its end real ones, through one thread per
+    ray, the nearest parts with their re-walk, and the lane walks. 86 GB of rays and hits."""
+    import torch
+    n, real = (1 << 31) + 77, 300
+    if torch.cuda.mem_get_info()[0] < 40 * n + (8 << 30):
+        pytest.skip("needs 94 GB of device memory")
+    rays = torch.zeros((n, 8), dtype=torch.float32, device="cuda")
+    rays[:, 3] = -1.0
+    ids, t = torch.empty(n, dtype=torch.int32, device="cuda"), torch.empty(n, dtype=torch.float32, device="cuda")
+    small, large = make_scene(rb.SCENE_CORNELL), make_scene(rb.SCENE_CITY, 0, 200_000)
+    for setup, kind in ((small, rb.TRACE_CLOSEST), (large, rb.TRACE_CLOSEST_QUEUE), (large, rb.TRACE_CLOSEST_STACKLESS),
+                        (large, rb.TRACE_ANY)):
+        host = seeded_rays(setup, real, seed=10)
+        rays[n - real:] = torch.from_numpy(host).cuda()
+        want, distance = np.zeros(real, np.int32), np.zeros(real, np.float32)
+        ob.load().oracle_trace(None, setup.host_scene(), host.ctypes.data, want.ctypes.data, distance.ctypes.data, real, kind)
+        ids.fill_(7)
+        t.fill_(7.0)
+        rb.check(rb.load().restir_trace(None, setup.device_scene(), rays.data_ptr(), ids.data_ptr(), t.data_ptr(), n, kind,
+                                        None), "restir_trace")
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(ids[n - real:].cpu().numpy(), want)
+        np.testing.assert_array_equal(t[n - real:].cpu().numpy().view(np.uint32), distance.view(np.uint32))
+        assert ids[:n - real].min() == -1 and ids[:n - real].max() == -1
+        assert t[:n - real].min() == -1.0 and t[:n - real].max() == -1.0
+    rb.status_flags()
+    del rays, ids, t
+    torch.cuda.empty_cache()
