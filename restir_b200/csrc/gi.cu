@@ -1387,8 +1387,9 @@ int residentBlocks(Kernel kernel, int threads, uint32_t blocksPerSm)
 	return sms * (blocksPerSm > 0u && int(blocksPerSm) < fit ? int(blocksPerSm) : fit);
 }
 
+// The launchers leave the launch status for the entry point to return at its end.
 template<bool kWide, int kThreads>
-int launchNearest(const BvhView& bvh, const RayQueue& q, uint32_t blocksPerSm, cudaStream_t s)
+void launchNearest(const BvhView& bvh, const RayQueue& q, uint32_t blocksPerSm, cudaStream_t s)
 {
 	static const int most = residentBlocks(traceQueueKernel<kWide, kThreads>, kThreads, 0u);
 	static const int mostRewalk = residentBlocks(rewalkQueueKernel<kWide, kThreads>, kThreads, 0u);
@@ -1396,22 +1397,19 @@ int launchNearest(const BvhView& bvh, const RayQueue& q, uint32_t blocksPerSm, c
 	const int limit = blocksPerSm > 0u ? int(min(blocksPerSm, 32u)) * sms : most;
 	traceQueueKernel<kWide, kThreads><<<min(limit, most), kThreads, 0, s>>>(bvh, q);
 	rewalkQueueKernel<kWide, kThreads><<<mostRewalk, kThreads, 0, s>>>(bvh, q);
-	return launchStatus();
 }
 
 template<int kThreads = 128>
-int launchQueueTracer(const BvhView& bvh, const RayQueue& q, cudaStream_t s, uint32_t blocksPerSm = 0u)
+void launchQueueTracer(const BvhView& bvh, const RayQueue& q, cudaStream_t s, uint32_t blocksPerSm = 0u)
 {
-	return wideRows(bvh) ? launchNearest<true, kThreads>(bvh, q, blocksPerSm, s)
-		: launchNearest<false, kThreads>(bvh, q, blocksPerSm, s);
+	wideRows(bvh) ? launchNearest<true, kThreads>(bvh, q, blocksPerSm, s) : launchNearest<false, kThreads>(bvh, q, blocksPerSm, s);
 }
 
 template<bool kWide, int kLanes>
-int launchWalk(const BvhView& bvh, const RayQueue& q, cudaStream_t s)
+void launchWalk(const BvhView& bvh, const RayQueue& q, cudaStream_t s)
 {
 	static const int blocks = residentBlocks(walkQueueKernel<kWide, kLanes>, 128, 0u);
 	walkQueueKernel<kWide, kLanes><<<blocks, 128, 0, s>>>(bvh, q);
-	return launchStatus();
 }
 
 // Four lanes a ray while the queue may hold at most two rays for each lane of
@@ -1420,9 +1418,9 @@ int launchWalk(const BvhView& bvh, const RayQueue& q, cudaStream_t s)
 // that: the 1080p frame, whose other passes run beside this one, takes 8.93
 // against 9.18 ms.
 template<bool kWide>
-int launchQueueWalk(const BvhView& bvh, const RayQueue& q, cudaStream_t s)
+void launchQueueWalk(const BvhView& bvh, const RayQueue& q, cudaStream_t s)
 {
-	return q.capacity <= 148u * 32u * 32u * 2u ? launchWalk<kWide, 4>(bvh, q, s) : launchWalk<kWide, 1>(bvh, q, s);
+	q.capacity <= 148u * 32u * 32u * 2u ? launchWalk<kWide, 4>(bvh, q, s) : launchWalk<kWide, 1>(bvh, q, s);
 }
 
 // The specular wavefront's workspace: [3 counters][rays 32 B x n][hit triangles
@@ -1668,14 +1666,18 @@ extern "C" int restir_trace_queue(const RestirScene* scene, void* queue, uint32_
 	switch (threads)
 	{
 	case 64:
-		return launchQueueTracer<64>(bvh, q, s, blocks_per_sm);
+		launchQueueTracer<64>(bvh, q, s, blocks_per_sm);
+		break;
 	case 128:
-		return launchQueueTracer<128>(bvh, q, s, blocks_per_sm);
+		launchQueueTracer<128>(bvh, q, s, blocks_per_sm);
+		break;
 	case 256:
-		return launchQueueTracer<256>(bvh, q, s, blocks_per_sm);
+		launchQueueTracer<256>(bvh, q, s, blocks_per_sm);
+		break;
 	default:
 		return RESTIR_ERROR_INVALID_ARGUMENT;
 	}
+	return launchStatus();
 }
 
 extern "C" int restir_gi_temporal_shade(const RestirParams* params, const RestirScene* scene, const RestirGBuffer* gbuffer,

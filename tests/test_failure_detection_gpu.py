@@ -178,3 +178,28 @@ def test_tensor_core_wait_gives_up_and_returns():
     assert torch.isfinite(out.float()).all()
     assert rb.status_flags() == 0
     assert lib.restir_cache_wait_check(0, result.data_ptr(), None) == rb.ERROR_INVALID_ARGUMENT
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("name, cache", [("gi_temporal", 0), ("gi_specular", 0), ("gi_temporal", 1), ("cache_train", 1)])
+def test_passes_with_a_queue_report_an_earlier_failure(name, cache):
+    """A call of several launches returns the failure of any of them, the queue tracer in its middle included. The
+    failure is made on the host: a frame of 2^40 pixels, whose first target cannot be allocated, leaves CUDA's last
+    error set, which the next call reports."""
+    import torch
+    from oracle.frame import FrameRunner
+    setup = make_scene(rb.SCENE_CORNELL)
+    setup.settings.radiance_cache = cache
+    setup.settings.cache_training_samples = 512
+    runner = FrameRunner(setup, 48, 48, "cuda", setup.settings, gi_wavefront=True)
+    runner.render()
+    runner.prepare()
+    run = dict(runner.passes())[name]
+    renderer = rb.Renderer(setup.settings)
+    renderer.set_scene(setup.mesh)
+    with pytest.raises(RuntimeError):
+        renderer.render(rb.frame_input(setup.mesh, 1 << 20, 1 << 20))
+    with pytest.raises(RuntimeError):
+        run()
+    run()  # and only once
+    torch.cuda.synchronize()
