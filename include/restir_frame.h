@@ -234,8 +234,8 @@ int restir_renderer_load_state(void* renderer, const char* path);
 
 /* Several views of one scene (each with its own camera and resolution)
  * rendered as one frame: the scene is uploaded once, the shadow atlas drawn
- * once, the GI candidate rays of every view go to one ray queue that a single
- * persistent tracer launch drains (restir_trace_queue), and the whole frame
+ * once, the GI candidate rays of every view go to one ray queue that one
+ * persistent tracer drains (restir_trace_queue), and the whole frame
  * is one CUDA graph whose per-view branches run on their own streams. Each
  * view's output equals a renderer's for that view alone. The radiance cache
  * is not available in a batch (settings.radiance_cache is ignored). */

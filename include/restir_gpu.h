@@ -262,7 +262,7 @@ uint64_t restir_gi_temporal_workspace_bytes(const RestirParams* params);
 /* restir_gi_temporal as a wavefront, with identical outputs: a candidates
  * pass (directions and depth-buffer marches) appends the rays it cannot
  * answer to a queue in the workspace, a persistent tracer walks the queue
- * (a lane takes the next ray as soon as its own finishes), and a shading
+ * (lanes whose rays have ended take the next ones), and a shading
  * pass completes cs_restir_temporal.sc from the recorded hits. workspace:
  * 256-byte aligned device memory of at least
  * restir_gi_temporal_workspace_bytes; it must not be shared with a call
@@ -274,7 +274,7 @@ int restir_gi_temporal_wavefront(const RestirParams* params, const RestirScene* 
 
 /* No reference counterpart: the wavefront's three steps with a ray queue the
  * caller owns, so that several views can fill one queue and have it traced
- * by a single persistent launch (restir_batch_* does this):
+ * at once (restir_batch_* does this):
  *   restir_ray_queue_reset(queue)                         counters to zero
  *   restir_gi_temporal_candidates(view ..., records, queue)   per view
  *   restir_trace_queue(scene, queue, ...)                 once
@@ -283,8 +283,10 @@ int restir_gi_temporal_wavefront(const RestirParams* params, const RestirScene* 
  * restir_ray_queue_bytes(capacity) bytes, capacity >= the sum of the views'
  * GI pixels x initial_candidates (rays past it are not traced: status bit
  * 2). records: 256-byte aligned, restir_gi_candidate_records_bytes(params)
- * per view. restir_trace_queue's threads (64, 128 or 256 per block) and
- * blocks_per_sm (0: as many as fit) shape the resident grid. */
+ * per view. restir_trace_queue is two persistent launches, the nearest-first
+ * walk and the stackless re-walk of the rays whose short stack dropped
+ * entries; its threads (64, 128 or 256 per block) and blocks_per_sm (0: as
+ * many as fit) shape the resident grid of both. */
 uint64_t restir_ray_queue_bytes(uint32_t capacity);
 int restir_ray_queue_reset(void* queue, void* stream);
 uint64_t restir_gi_candidate_records_bytes(const RestirParams* params);
@@ -354,8 +356,8 @@ uint64_t restir_gi_specular_workspace_bytes(const RestirParams* params);
 /* restir_gi_specular as a wavefront, with identical outputs: a rays pass
  * (reflection directions and depth-buffer marches) appends the rays the
  * march does not answer to a queue in the workspace, a persistent tracer
- * runs the stackless walk over the queue (a lane takes the next ray as soon
- * as its own ends), and a shading pass completes fs_specular.sc from the
+ * runs the stackless walk over the queue (lanes, or groups of four, whose
+ * rays have ended take the next ones), and a shading pass completes fs_specular.sc from the
  * recorded hits. workspace: 256-byte aligned device memory of at least
  * restir_gi_specular_workspace_bytes; it must not be shared with a call
  * whose kernels may overlap this one's. */

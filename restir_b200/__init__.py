@@ -587,7 +587,7 @@ class RadianceCache:
 class Batch:
     """Several views of one scene rendered as one frame (include/restir_frame.h,
     restir_batch_*): one scene upload, one shadow atlas, one GI ray queue
-    traced by a single persistent launch, one CUDA graph per frame."""
+    traced by one persistent tracer, one CUDA graph per frame."""
 
     def __init__(self, settings: RestirSettings | None, views: int):
         self._lib = load()

@@ -537,7 +537,7 @@ __global__ void __launch_bounds__(128, RESTIR_GI_SPATIAL_MIN_BLOCKS) giSpatialKe
 //
 // A: candidate directions and depth-buffer marches; the rays the march cannot
 //    answer go to a ray queue (warp-vote compaction).
-// B: the persistent closest-hit tracer over the queue (wavefront.cuh).
+// B: the persistent closest-hit tracer over the queue and its re-walk (wavefront.cuh).
 // C: the rest of cs_restir_temporal.sc, reading A's and B's results where
 //    the megakernel traced; the random stream is replayed from the pixel's
 //    seed, so every number is the megakernel's.
@@ -1369,34 +1369,45 @@ TemporalWorkspace layoutTemporalWorkspace(const RestirParams* p, void* base)
 	return w;
 }
 
-// One resident grid of a queue tracer: SMs x blocks that fit on one SM (or
-// blocksPerSm, when that is fewer), looked up once per kernel (not inside a
-// stream capture on later calls).
-template<typename Kernel>
-int residentBlocks(Kernel kernel, int threads, uint32_t blocksPerSm)
+// The resident grid of a queue tracer's kernel: the SMs and the blocks that fit
+// on one, looked up once per kernel (not inside a stream capture on later calls).
+struct ResidentGrid
 {
-	int device = 0, sms = 148, fit = 0;
+	int sms = 148, perSm = 0;
+
+	// blocksPerSm: at most so many on one SM (0: as many as fit).
+	int blocks(uint32_t blocksPerSm = 0u) const
+	{
+		return sms * (blocksPerSm > 0u && blocksPerSm < uint32_t(perSm) ? int(blocksPerSm) : perSm);
+	}
+};
+
+template<typename Kernel>
+ResidentGrid residentGrid(Kernel kernel, int threads)
+{
+	ResidentGrid grid;
+	int device = 0;
 	if (cudaGetDevice(&device) == cudaSuccess)
 	{
-		cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+		cudaDeviceGetAttribute(&grid.sms, cudaDevAttrMultiProcessorCount, device);
 	}
-	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel, threads, 0) != cudaSuccess || fit < 1)
+	if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&grid.perSm, kernel, threads, 0) != cudaSuccess || grid.perSm < 1)
 	{
-		fit = 1;
+		grid.perSm = 1;
 	}
-	return sms * (blocksPerSm > 0u && int(blocksPerSm) < fit ? int(blocksPerSm) : fit);
+	return grid;
 }
 
-// The launchers leave the launch status for the entry point to return at its end.
+// Both launches keep to blocksPerSm: the re-walk takes about as long as the
+// first. The launchers leave the launch status for the entry point to return at
+// its end.
 template<bool kWide, int kThreads>
 void launchNearest(const BvhView& bvh, const RayQueue& q, uint32_t blocksPerSm, cudaStream_t s)
 {
-	static const int most = residentBlocks(traceQueueKernel<kWide, kThreads>, kThreads, 0u);
-	static const int mostRewalk = residentBlocks(rewalkQueueKernel<kWide, kThreads>, kThreads, 0u);
-	static const int sms = residentBlocks(traceQueueKernel<kWide, kThreads>, kThreads, 1u);
-	const int limit = blocksPerSm > 0u ? int(min(blocksPerSm, 32u)) * sms : most;
-	traceQueueKernel<kWide, kThreads><<<min(limit, most), kThreads, 0, s>>>(bvh, q);
-	rewalkQueueKernel<kWide, kThreads><<<mostRewalk, kThreads, 0, s>>>(bvh, q);
+	static const ResidentGrid nearest = residentGrid(traceQueueKernel<kWide, kThreads>, kThreads);
+	static const ResidentGrid rewalk = residentGrid(rewalkQueueKernel<kWide, kThreads>, kThreads);
+	traceQueueKernel<kWide, kThreads><<<nearest.blocks(blocksPerSm), kThreads, 0, s>>>(bvh, q);
+	rewalkQueueKernel<kWide, kThreads><<<rewalk.blocks(blocksPerSm), kThreads, 0, s>>>(bvh, q);
 }
 
 template<int kThreads = 128>
@@ -1408,8 +1419,8 @@ void launchQueueTracer(const BvhView& bvh, const RayQueue& q, cudaStream_t s, ui
 template<bool kWide, int kLanes>
 void launchWalk(const BvhView& bvh, const RayQueue& q, cudaStream_t s)
 {
-	static const int blocks = residentBlocks(walkQueueKernel<kWide, kLanes>, 128, 0u);
-	walkQueueKernel<kWide, kLanes><<<blocks, 128, 0, s>>>(bvh, q);
+	static const ResidentGrid walk = residentGrid(walkQueueKernel<kWide, kLanes>, 128);
+	walkQueueKernel<kWide, kLanes><<<walk.blocks(), 128, 0, s>>>(bvh, q);
 }
 
 // Four lanes a ray while the queue may hold at most two rays for each lane of
@@ -1546,7 +1557,7 @@ extern "C" int restir_gi_specular_wavefront(const RestirParams* params, const Re
 // --- the wavefront's three steps with a caller-owned, shareable ray queue ---------
 //
 // Several views (or frames) can append to one queue and have it traced by a
-// single persistent launch: restir_gi_temporal_candidates for each, one
+// persistent tracer: restir_gi_temporal_candidates for each, one
 // restir_trace_queue, restir_gi_temporal_shade for each.
 
 namespace restir

@@ -1346,8 +1346,8 @@ private:
 
 // Several views of one scene rendered as one frame (no reference
 // counterpart): the views share the scene's buffers, one shadow atlas (it
-// depends on the light and the scene only) and one GI ray queue that a single
-// persistent tracer launch drains; the frame is captured as one CUDA graph in
+// depends on the light and the scene only) and one GI ray queue that one
+// persistent tracer drains; the frame is captured as one CUDA graph in
 // which each view's passes run on its own stream, so that small views fill
 // the GPU together. Every view's output equals what a Renderer of that view
 // alone produces.

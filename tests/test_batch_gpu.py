@@ -98,3 +98,34 @@ def test_trace_queue_shapes_bit_exact(threads, blocks):
     np.testing.assert_array_equal(got_ids, ids)
     np.testing.assert_array_equal(got_t.view(np.uint32), t.view(np.uint32))
     assert lib.restir_trace_queue(setup.device_scene(), queue.data_ptr(), n, 96, 0, None) == rb.ERROR_INVALID_ARGUMENT
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("threads", [64, 128, 256])
+@pytest.mark.parametrize("offset", [0, 4])
+def test_blocks_per_sm_limits_every_launch(threads, offset):
+    """Every launch of restir_trace_queue keeps to blocks_per_sm, read from the grids of the captured launches."""
+    import torch
+    from cuda.bindings import driver
+    setup = make_scene(rb.SCENE_CORNELL)
+    scene = setup.device_scene()
+    rows = torch.zeros(setup.bvh.data.size + 4, dtype=torch.float32, device="cuda")
+    rows[offset:offset + setup.bvh.data.size] = torch.from_numpy(setup.bvh.data).cuda()
+    scene.bvh = rows[offset:].data_ptr()
+    queue = torch.zeros(int(rb.load().restir_ray_queue_bytes(1000)), dtype=torch.uint8, device="cuda")
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+
+    def grids(blocks):
+        graph = torch.cuda.CUDAGraph(keep_graph=True)
+        with torch.cuda.graph(graph):
+            stream = torch.cuda.current_stream().cuda_stream
+            rb.check(rb.load().restir_trace_queue(scene, queue.data_ptr(), 1000, threads, blocks, stream), "trace_queue")
+        raw = driver.CUgraph(graph.raw_cuda_graph())
+        _, _, count = driver.cuGraphGetNodes(raw)
+        _, nodes, _ = driver.cuGraphGetNodes(raw, count)
+        return [driver.cuGraphKernelNodeGetParams(node)[1].gridDimX for node in nodes]
+
+    most = grids(0)
+    assert len(most) == 2 and all(g >= 2 * sms for g in most)
+    for blocks in (1, 2, 64):
+        assert grids(blocks) == [min(blocks * sms, g) for g in most], blocks
