@@ -162,7 +162,6 @@ __device__ __forceinline__ void boilAndStore(const RestirParams& P, const GiPass
 // cs_restir_temporal.sc:192-296 after the fresh candidates: temporal reuse
 // with pairwise MIS, the boiling filter over the warp's 4x8 group, the
 // reservoir stores. Every lane of the warp must call it (the group sum).
-template<bool kWave>
 __device__ __forceinline__ void temporalReuseAndStore(const RestirParams& P, const GiPass& g, const GiBindings& b, int lane,
 	bool inside, bool working, int px, int py, V3 position, V3 normal, V3 albedo, const GiReservoir& canonical, uint32_t rng)
 {
@@ -177,6 +176,7 @@ __device__ __forceinline__ void temporalReuseAndStore(const RestirParams& P, con
 	const float radius = g.reuseRadius(position);
 	PairwiseMis mis = g.beginPairwiseMis(position, normal, canonical, canonical.count, P.temporal_taps);
 	float combinedWeight = 0.0f;
+	const unsigned workers = __ballot_sync(0xffffffffu, working);
 	if (working)
 	{
 		for (int tapIndex = 0; tapIndex < P.temporal_taps; ++tapIndex)
@@ -210,20 +210,54 @@ __device__ __forceinline__ void temporalReuseAndStore(const RestirParams& P, con
 					f4(__ldg(b.historyNormal + i)), position, normal, radius, neighbour);
 				neighbour.cacheSlot = g.cache != nullptr ? g.cacheNeighbourBase + i : -1;
 			}
-			if (!accepted)
+			float neighbourGeometry = 0.0f;
+			bool test = false;
+			if (accepted)
+			{
+				test = g.neighbourBegin(mis, neighbour, neighbourGeometry);
+			}
+			else
 			{
 				GiPass::skipNeighbour(mis);
-				continue;
 			}
-			g.template addNeighbour<kWave>(mis, position, normal, albedo, neighbour, randomSelect);
+			__syncwarp(workers);
+			const bool occluded = test && !g.isVisible<kWalkEither>(neighbour.receiverPosition, neighbour.receiverNormal,
+				mis.canonicalPosition, mis.canonicalId);
+			__syncwarp(workers);
+			if (accepted)
+			{
+				g.neighbourShare(mis, neighbour, neighbourGeometry, occluded);
+				V3 contribution = v3s(0.0f);
+				V3 sampleNormal = v3(0.0f, 0.0f, 1.0f);
+				bool shifted = false;
+				if (neighbour.weight > 0.0f)
+				{
+					shifted = g.evaluateSample(position, normal, albedo, neighbour.samplePosition, neighbour.sampleId, contribution,
+						sampleNormal, neighbour.cacheSlot);
+				}
+				g.neighbourShift(mis, position, normal, neighbour, shifted, contribution, sampleNormal, randomSelect);
+			}
 		}
-		combinedWeight = g.template finishPairwiseMis<kWave>(mis, position, normal, canonical, canonicalWeight, nextRandom(rng));
+		const bool test = g.finishBegin(mis, canonical, canonicalWeight, nextRandom(rng), combinedWeight);
+		__syncwarp(workers);
+		if (test && !g.isVisible<kWalkEither>(position, normal, mis.combined.position, mis.combined.id))
+		{
+			combinedWeight = 0.0f;
+		}
 	}
 	boilAndStore(P, g, b, lane, inside, working, px, py, position, normal, albedo, canonical, canonicalWeight, previousUv, mis,
 		combinedWeight);
 }
 
-template<bool kWave>
+// The pass as one kernel. Bound by divergence and instruction fetch: a warp's
+// lanes join before each walk and each evaluation, and both visibility walks
+// are in it (kWalkEither). us at 320x180 / 640x360 in the 100k-triangle city,
+// 1280x720 with half-size GI in the courtyard, 960x540 in the 1M-triangle city,
+// BVH rays: lane walk 602 / 1,008 / 851 / 2,152, lock step 680 / 1,118 / 1,024
+// / 2,243. An instance for each walk without the joins: 689 / 1,132 / 917 /
+// 2,283 and 902 / 1,359 / 1,261 / 2,553; with them: 642 / 1,091 / 869 / 2,217
+// and 816 / 1,251 / 1,146 / 2,398. Both in one expression instead of two returns
+// (isVisible): 676 / 1,137 / 928 / 2,269 and 799 / 1,247 / 1,145 / 2,393.
 __global__ void __launch_bounds__(kGiThreads, RESTIR_GI_TEMPORAL_MIN_BLOCKS) giTemporalKernel(const RestirParams P, BvhView bvh,
 	GiBindings b)
 {
@@ -267,6 +301,7 @@ __global__ void __launch_bounds__(kGiThreads, RESTIR_GI_TEMPORAL_MIN_BLOCKS) giT
 			hit = g.traceScreenSpaceRay(rayOrigin, direction, g.kMaxRayDistance(), hitPosition);
 		}
 		bool needBvh = working && !hit && P.ray_mode != RESTIR_RAY_MODE_SCREEN;
+		__syncwarp();
 		if (needBvh)
 		{
 			float queueDistance;
@@ -288,6 +323,7 @@ __global__ void __launch_bounds__(kGiThreads, RESTIR_GI_TEMPORAL_MIN_BLOCKS) giT
 		V3 contribution = v3s(0.0f);
 		V3 hitNormal = v3s(0.0f);
 		bool evaluated = false;
+		__syncwarp();
 		if (hit)
 		{
 			evaluated = g.evaluateSample(position, normal, albedo, hitPosition, hitId, contribution, hitNormal);
@@ -315,7 +351,7 @@ __global__ void __launch_bounds__(kGiThreads, RESTIR_GI_TEMPORAL_MIN_BLOCKS) giT
 		}
 	}
 
-	temporalReuseAndStore<kWave>(P, g, b, lane, inside, working, px, py, position, normal, albedo, canonical, rng);
+	temporalReuseAndStore(P, g, b, lane, inside, working, px, py, position, normal, albedo, canonical, rng);
 }
 
 template<bool kWave>
@@ -447,7 +483,7 @@ __global__ void __launch_bounds__(128, RESTIR_GI_SPATIAL_MIN_BLOCKS) giSpatialKe
 			toId = mis.combined.id;
 		}
 		__syncthreads();
-		const bool occluded = test && !g.template isVisible<kWave>(from, fromNormal, to, toId);
+		const bool occluded = test && !g.template isVisible<kWave ? kWalkWarp : kWalkLane>(from, fromNormal, to, toId);
 		if (tapIndex == taps)
 		{
 			if (occluded)
@@ -797,7 +833,7 @@ __global__ void __launch_bounds__(kGiThreads, RESTIR_GI_TEMPORAL_MIN_BLOCKS) giT
 			toId = mis.combined.id;
 		}
 		__syncthreads();
-		const bool occluded = test && !g.template isVisible<kWave>(from, fromNormal, to, toId);
+		const bool occluded = test && !g.template isVisible<kWave ? kWalkWarp : kWalkLane>(from, fromNormal, to, toId);
 		if (step == candidates + taps)
 		{
 			if (occluded)
@@ -1242,7 +1278,7 @@ extern "C" int restir_gi_temporal(const RestirParams* params, const RestirScene*
 	b.outReceiver = reinterpret_cast<float4*>(output->receiver);
 	b.outNormal = reinterpret_cast<float4*>(output->normal);
 	const int groups = int((params->gi_width + 3) / 4 * ((params->gi_height + 7) / 8));
-	(params->wave_visibility > 0.5f ? giTemporalKernel<true> : giTemporalKernel<false>)<<<(groups + kGiWarps - 1) / kGiWarps, kGiThreads, 0, asStream(stream)>>>(*params, makeBvhView(scene), b);
+	giTemporalKernel<<<(groups + kGiWarps - 1) / kGiWarps, kGiThreads, 0, asStream(stream)>>>(*params, makeBvhView(scene), b);
 	return launchStatus();
 }
 

@@ -185,6 +185,10 @@ __device__ __forceinline__ V3 skyRadiance(const RestirParams& P, V3 d)
 	return height >= 0.0f ? mix(horizon, zenith, sqrtf(height)) : mix(horizon, ground, sqrtf(-height));
 }
 
+// Which visibility walk a kernel holds (traceVisibility): the lanes' own, the
+// warp's in lock step, or both with wave_visibility deciding between them.
+constexpr int kWalkLane = 0, kWalkWarp = 1, kWalkEither = 2;
+
 // The resources a GI pass binds (renderer.cpp:772-802) and restir.sh's
 // functions over them.
 struct GiPass
@@ -575,7 +579,7 @@ struct GiPass
 		return receiverCosine > 0.0f && sampleCosine > 0.0f ? receiverCosine * sampleCosine / distanceSquared : 0.0f;
 	}
 
-	template<bool kWave>
+	template<int kWalk>
 	__device__ inline bool isVisible(V3 receiverPosition, V3 receiverNormal, V3 samplePosition, float sampleId) const
 	{
 		V3 origin = receiverPosition + receiverNormal * kRayBias();
@@ -589,8 +593,13 @@ struct GiPass
 		if (bvhRay)
 		{
 			float occluderDistance = 0.0f;
-			return traceVisibility<kWave>(bvh, origin, direction, sky ? kMaxBvhRayDistance() : sampleDistance - kRayBias(),
-				occluderDistance) < 0;
+			const float reach = sky ? kMaxBvhRayDistance() : sampleDistance - kRayBias();
+			const bool warpWalk = kWalk == kWalkEither ? P.wave_visibility > 0.5f : kWalk == kWalkWarp;
+			if (warpWalk)
+			{
+				return traceVisibility<true>(bvh, origin, direction, reach, occluderDistance) < 0;
+			}
+			return traceVisibility<false>(bvh, origin, direction, reach, occluderDistance) < 0;
 		}
 		if (sky)
 		{
@@ -673,10 +682,10 @@ struct GiPass
 		mis.canonicalShare += mis.pairCanonical;
 	}
 
-	// addNeighbour and finishPairwiseMis in parts around their visibility test
-	// and sample evaluation, so that a kernel can run all of its reuse's tests
-	// and evaluations at one call site each (its code then fits the
-	// instruction cache); the arithmetic is the same either way.
+	// Pairwise MIS in parts around its visibility tests and sample evaluations,
+	// so that a kernel can bring a warp's lanes together before each, and run
+	// all of them at one call site each (its code then fits the instruction
+	// cache).
 	//
 	// Neighbour, part 1: the count, and the canonical sample's geometry term
 	// at the neighbour; true when that term needs the visibility test from the
@@ -735,26 +744,6 @@ struct GiPass
 		}
 	}
 
-	template<bool kWave>
-	__device__ inline void addNeighbour(PairwiseMis& mis, V3 p, V3 n, V3 albedo, const NeighbourReservoir& nb, float random) const
-	{
-		float neighbourGeometry;
-		bool occluded = false;
-		if (neighbourBegin(mis, nb, neighbourGeometry))
-		{
-			occluded = !isVisible<kWave>(nb.receiverPosition, nb.receiverNormal, mis.canonicalPosition, mis.canonicalId);
-		}
-		neighbourShare(mis, nb, neighbourGeometry, occluded);
-		V3 contribution = v3s(0.0f);
-		V3 sampleNormal = v3(0.0f, 0.0f, 1.0f);
-		bool shifted = false;
-		if (nb.weight > 0.0f)
-		{
-			shifted = evaluateSample(p, n, albedo, nb.samplePosition, nb.sampleId, contribution, sampleNormal, nb.cacheSlot);
-		}
-		neighbourShift(mis, p, n, nb, shifted, contribution, sampleNormal, random);
-	}
-
 	// The combination, part 1: the canonical sample's update and the combined
 	// weight; true when a chosen neighbour's sample needs the visibility test
 	// from this pixel (part 2: a failed test zeroes the weight).
@@ -774,21 +763,6 @@ struct GiPass
 			? mis.combined.weightSum / (mis.totalCount * mis.combined.target)
 			: 0.0f;
 		return combinedWeight > 0.0f && mis.neighbourSelected;
-	}
-
-	template<bool kWave>
-	__device__ inline float finishPairwiseMis(PairwiseMis& mis, V3 p, V3 n, const GiReservoir& canonical, float canonicalWeight,
-		float random) const
-	{
-		float combinedWeight;
-		if (finishBegin(mis, canonical, canonicalWeight, random, combinedWeight))
-		{
-			if (!isVisible<kWave>(p, n, mis.combined.position, mis.combined.id))
-			{
-				combinedWeight = 0.0f;
-			}
-		}
-		return combinedWeight;
 	}
 };
 
