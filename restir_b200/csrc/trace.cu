@@ -16,23 +16,36 @@ namespace
 constexpr int kTraceBlock = 128;
 
 // Which kernel traces a ray set, by its size n and the scene's nodes. Measured
-// on random rays (us; one thread a ray / four lanes a ray / warp with leaves
-// tested together):
-//   any hit, 1M-triangle city, n 1,000: 81 / 47 / 87; 16,000: 105 / 75 / 129;
-//     64,000: 109 / 119 / 136; 400,000: 282 / 336 / 208;
-//   any hit, Cornell box, 16,000: 21 / 15 / 23; 400,000: 54 / 77 / 60;
-//   stackless, city, 16,000: 812 / 587 / 978; 1,000,000: - / 4,080 / 2,490;
-//   closest, city, 1,000: 378 / - / 320; 400,000: 1,247 / - / 1,018;
-//   closest, Cornell box, 1,000: 19 / - / 25; 400,000: 64 / - / 83.
-// So up to a group of four lanes for each ray that the SMs hold at once (148 x
-// 32 warps x 8), walks are latency-bound and take four lanes; until every lane
-// has two rays, one thread each is enough; past that, and for nearest hits,
-// the warp's shared leaves win, unless the scene is so small that a ray visits
-// some twenty nodes and half of the time goes to fetching the longer code.
-constexpr uint32_t kFourLaneRays = 148u * 32u * 8u;
-constexpr uint32_t kThreadRays = 148u * 32u * 32u * 2u;
-constexpr int kSmallScene = 4096;
+// on random rays, 43 to 1.9M nodes, n 1 to 1M (us; 4: four lanes a ray, 1: one
+// thread a ray, w: a warp's part, leaves tested together):
+//   any hit, city of 1.9M nodes, n 1,000: 4 47, 1 81, w 87; 64,000: 4 127, 1 142,
+//     w 127; 300,000: 4 250, 1 214, w 196; Cornell box, 16,000: 4 15, 1 21, w 23;
+//     64,000: 4 23, 1 21, w 18; 500,000: 4 87, 1 60, w 53;
+//   stackless, city of 47k nodes, 64,000: 4 158, 1 148, w 156; 200,000: 4 293,
+//     1 251, w 263; of 1.9M, 1,000,000: 1 3,762, w 2,502; Cornell box, 300,000:
+//     1 49, w 56; 500,000: 1 73, w 73;
+//   closest, city of 1.9M nodes, 1: 1 70, w 89; 1,000: 1 268, w 225; 1,000,000:
+//     1 2,325, w 1,813; of 190k, 32: 1 101, w 115; 200: 1 107, w 118; 200,000:
+//     1 396, w 410; of 47k, 16,000: 1 60, w 74; 300,000: 1 159, w 180; 500,000:
+//     1 216, w 215; of 10k, 1,000,000: 1 220, w 228.
+// So walks take four lanes up to a group of them for each ray that the SMs hold
+// at once (148 x 32 warps x 8), where they are latency-bound; then any hits take
+// the warp's shared leaves, stackless nearest hits one thread each until every
+// lane has two rays. Nearest hits take one thread each where a ray visits few
+// nodes or the rays are few: below 128, in scenes of up to 12,288 nodes always,
+// up to 131,072 nodes until every lane has three rays, and just past one ray a
+// lane, where the parts' last warps leave the SMs idle.
+constexpr uint32_t kResidentLanes = 148u * 32u * 32u;
+constexpr uint32_t kFourLaneRays = kResidentLanes / 4u;
+constexpr uint32_t kFewRays = 128u;
+constexpr int kSmallScene = 12288;
+constexpr int kMiddleScene = 131072;
 
+bool nearestPerThread(uint32_t n, int nodes)
+{
+	return n < kFewRays || nodes <= kSmallScene || (nodes <= kMiddleScene && n <= 3u * kResidentLanes)
+		|| (n > kResidentLanes && n <= kResidentLanes + kResidentLanes / 2u);
+}
 
 // A contiguous part of the ray set, one per warp: its lanes take the part's
 // rays as theirs end, without an atomic.
@@ -104,7 +117,7 @@ __global__ void __launch_bounds__(kTraceBlock, 8) walkPartsKernel(BvhView bvh, R
 }
 
 // One thread per ray, a kernel per kind (each fetches its own kind's code only:
-// 1,000 any-hit rays in the Cornell box take 21 us against 23 us in one kernel
+// 1,000 nearest hits in the Cornell box take 17 us against 21 us in one kernel
 // for all kinds).
 template<int kKind, bool kWide = false>
 __global__ void __launch_bounds__(kTraceBlock) traceKernel(BvhView bvh, RayArrays arrays, uint32_t n)
@@ -122,9 +135,9 @@ __global__ void __launch_bounds__(kTraceBlock) traceKernel(BvhView bvh, RayArray
 	{
 		r.hit = traceBvh(bvh, r.o, r.d, length, false, r.distance, stack + threadIdx.x, kTraceBlock);
 	}
-	else if (kKind == RESTIR_TRACE_ANY || kKind == RESTIR_TRACE_CLOSEST_STACKLESS)
+	else if (kKind == RESTIR_TRACE_CLOSEST_STACKLESS)
 	{
-		r.hit = traceBvh(bvh, r.o, r.d, length, kKind == RESTIR_TRACE_ANY, r.distance, nullptr, 0);
+		r.hit = traceBvh(bvh, r.o, r.d, length, false, r.distance, nullptr, 0);
 	}
 	else if (kKind == RESTIR_TRACE_ANY_WAVE)
 	{
@@ -149,7 +162,7 @@ void launchThreads(const BvhView& bvh, const RayArrays& arrays, uint32_t n, cuda
 // lanes whose rays end early have more to take.
 uint32_t partOf(uint32_t n, uint32_t takers)
 {
-	return n > 148u * 32u * takers ? 4u * takers : takers;
+	return n > kResidentLanes / 32u * takers ? 4u * takers : takers;
 }
 
 uint32_t partBlocks(uint32_t n, uint32_t part)
@@ -217,8 +230,6 @@ extern "C" int restir_trace(const RestirParams* params, const RestirScene* scene
 	BvhView bvh = makeBvhView(scene);
 	cudaStream_t s = asStream(stream);
 	const RayArrays arrays = { reinterpret_cast<const float4*>(rays), hit_triangle, hit_distance };
-	const bool small = bvh.nodeCount <= kSmallScene;
-	const bool threads = n > kFourLaneRays && (small || n <= kThreadRays);
 	if (kind == RESTIR_TRACE_ANY_WAVE)
 	{
 		launchThreads<RESTIR_TRACE_ANY_WAVE>(bvh, arrays, n, s);
@@ -234,15 +245,11 @@ extern "C" int restir_trace(const RestirParams* params, const RestirScene* scene
 			launchThreads<RESTIR_TRACE_CLOSEST_WATERTIGHT>(bvh, arrays, n, s);
 		}
 	}
-	else if (kind == RESTIR_TRACE_CLOSEST && small)
+	else if (kind == RESTIR_TRACE_CLOSEST && nearestPerThread(n, bvh.nodeCount))
 	{
 		launchThreads<RESTIR_TRACE_CLOSEST>(bvh, arrays, n, s);
 	}
-	else if (kind == RESTIR_TRACE_ANY && threads)
-	{
-		launchThreads<RESTIR_TRACE_ANY>(bvh, arrays, n, s);
-	}
-	else if (kind == RESTIR_TRACE_CLOSEST_STACKLESS && threads)
+	else if (kind == RESTIR_TRACE_CLOSEST_STACKLESS && n > kFourLaneRays && n <= 2u * kResidentLanes)
 	{
 		launchThreads<RESTIR_TRACE_CLOSEST_STACKLESS>(bvh, arrays, n, s);
 	}
