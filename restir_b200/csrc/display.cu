@@ -23,7 +23,8 @@ namespace
 // start to end, and by fetching them: large blocks, whose barrier keeps 16 warps
 // in the same part of them, took 0.263 ms at 2560x1440 (0.049 at 960x540) where
 // blocks of 128 and of 256 threads took 0.312 and 0.302 (0.058, 0.056), and 2
-// blocks of 512 0.291 (0.053).
+// blocks of 512 0.291 (0.053), all with the exposure's scale computed by 13 of
+// the 16 warps; by one of them 0.251 (0.047).
 #ifndef RESTIR_DISPLAY_MIN_BLOCKS
 #define RESTIR_DISPLAY_MIN_BLOCKS 3
 #endif
@@ -390,7 +391,7 @@ __device__ __forceinline__ void storeBytes(uint8_t* p, size_t i, uint32_t r, uin
 __device__ __forceinline__ float exposureScale(const RestirDisplayParams& P, const uint32_t* __restrict__ exposure)
 {
 	float scale = rn_exp2(P.exposure_ev);
-	if (P.auto_exposure > 0.5f && P.pass_through <= 0.5f)
+	if (P.auto_exposure > 0.5f)
 	{
 		scale = scale * (0.18f / rn_exp2(__uint_as_float(*exposure)));
 	}
@@ -442,11 +443,15 @@ __global__ void __launch_bounds__(kTileW * kTileH, RESTIR_DISPLAY_MIN_BLOCKS) di
 	__shared__ float4 tile[kHaloW * kHaloH];
 	__shared__ float sharedScale;
 	const int W = int(P.width), H = int(P.height);
-	if ((kMode & kModeTonemap) && threadIdx.x >= 96u)
+	// One warp for the block, the last, which has no texel of the border: the two
+	// powers are 4% of a pixel's instructions. Not for the views that show a
+	// colour as it is.
+	const bool scaled = (kMode & kModeTonemap) != 0 && P.pass_through <= 0.5f && P.reference_view <= 1.5f;
+	constexpr unsigned kScaleThread = kTileW * kTileH - 32;
+	if (scaled && threadIdx.x >= kScaleThread)
 	{
-		// One warp for the block: the two powers are 4% of a pixel's instructions.
 		const float scale = exposureScale(P, exposure);
-		if (threadIdx.x == 96u)
+		if (threadIdx.x == kScaleThread)
 		{
 			sharedScale = scale;
 		}
@@ -460,7 +465,10 @@ __global__ void __launch_bounds__(kTileW * kTileH, RESTIR_DISPLAY_MIN_BLOCKS) di
 	{
 		loadNeighbourhood(tile, hdr, depth, W, H, int(blockIdx.x) * kTileW, int(blockIdx.y) * kTileH, lx, ly, current, compressed);
 	}
-	__syncthreads();
+	if ((kMode & kModeTaa) || scaled)
+	{
+		__syncthreads();
+	}
 	if (x >= W || y >= H)
 	{
 		return;
