@@ -221,3 +221,23 @@ def test_display_tile_edges(size):
     rb.check(rb.load().restir_taa(C.byref(p), hdr.data_ptr(), depth.data_ptr(), history.data_ptr(), out.data_ptr(), None),
              "restir_taa")
     np.testing.assert_array_equal(host(out), expected)
+
+
+@pytest.mark.parametrize("size", [(1, 1), (127, 1), (129, 1), (43, 3)])
+@pytest.mark.parametrize("view, through", [(2.0, 0.0), (0.0, 1.0), (1.0, 1.0), (2.0, 1.0)])
+def test_plain_views_at_block_edges(size, view, through):
+    """The views without an operator (one pixel a thread, 128 a block): below a block, one more, and several rows."""
+    w, h = size
+    rng = np.random.default_rng(w)
+    inputs = display_inputs(w, h, seed=w, specials=False)
+    mean = rng.lognormal(-1.0, 1.5, (3, w * h))
+    alpha = (rng.random(w * h) < 0.8).astype(np.uint8)
+    p = display_params(w, h, inputs, reference_view=view, pass_through=through, auto_exposure=0.0)
+    expected = np.zeros(w * h * 4, np.uint8)
+    ob.load().oracle_tonemap(C.byref(p), inputs["hdr"].ctypes.data, None, mean.ctypes.data, alpha.ctypes.data,
+                             expected.ctypes.data)
+    hdr, mean_d, alpha_d = device(inputs["hdr"]), device(mean), device(alpha)
+    out = device(np.zeros(w * h * 4 + 4, np.uint8))
+    rb.check(rb.load().restir_tonemap(C.byref(p), hdr.data_ptr(), None, mean_d.data_ptr(), alpha_d.data_ptr(),
+                                      out.data_ptr(), None), "restir_tonemap")
+    np.testing.assert_array_equal(host(out), np.append(expected, np.zeros(4, np.uint8)))
