@@ -155,65 +155,42 @@ __device__ __forceinline__ float splineWeight(int offset)
 	return d == 0 ? 0.375f : (d == 1 ? 0.25f : 0.0625f);
 }
 
-// One a-trous level. A pixel's taps lie step texels apart, so the pixels of one
-// residue (x mod step, y mod step) filter among themselves: a block takes 16x8
-// of them, at any step, and its 20x12 texels go to shared memory once, the
-// normals normalised there. Every tap used to fetch 40 bytes and normalise the
-// neighbour's normal (a square root and a division, 24 times per texel instead
-// of 1.9) at 220 instructions a tap. Bound by issue (79% of the slots busy);
-// five levels at 960x540 take 0.36 ms, before 0.52 ms; the rows are a loop, so
-// that its 1,360 instructions stay in the instruction cache (unrolled: 0.42 ms).
-constexpr int kFilterTileW = kFilterW + 4, kFilterTileH = kFilterH + 4;
-
 struct FilterTexel
 {
 	GeometryTexel geometry;  // position.w: luminance
 	float4 color;            // w: variance
 };
 
-__global__ void __launch_bounds__(128) atrousKernel(const RestirParams P, int step, int residuesX, int residuesY,
-	int blocksX, const uint16_t* __restrict__ input, const float4* __restrict__ receiver, const float4* __restrict__ normal, uint16_t* out)
+// What a tap at (x, y) reads.
+__device__ __forceinline__ FilterTexel filterTexel(const uint16_t* __restrict__ input, const float4* __restrict__ receiver,
+	const float4* __restrict__ normal, int w, int h, int x, int y)
 {
-	__shared__ FilterTexel tile[kFilterTileW * kFilterTileH];
+	FilterTexel t = { outsideTexel(), make_float4(0.0f, 0.0f, 0.0f, 0.0f) };
+	if (x >= 0 && x < w && y >= 0 && y < h)
+	{
+		const V4 color = loadH4(input, y * w + x);
+		t.geometry = geometryTexel(receiver, normal, y * w + x, luminance(color.xyz()));
+		t.color = make_float4(color.x, color.y, color.z, color.w);
+	}
+	return t;
+}
+
+// One a-trous level's pixel (px, py) from its own texel and its taps',
+// tap(x, y) for offsets of -2 to 2 steps.
+template<typename Tap>
+__device__ __forceinline__ void filterPixel(const RestirParams& P, const uint16_t* __restrict__ input, uint16_t* out, int px, int py,
+	const GeometryTexel& center, Tap tap)
+{
 	const int w = int(P.gi_width), h = int(P.gi_height);
-	// Neighbouring blocks take neighbouring residues: they read the same lines.
-	const int blockX = int(blockIdx.x % uint32_t(blocksX)), blockY = int(blockIdx.x / uint32_t(blocksX));
-	const int firstX = blockX % residuesX + blockX / residuesX * kFilterW * step;
-	const int firstY = blockY % residuesY + blockY / residuesY * kFilterH * step;
-	if (firstX >= w || firstY >= h)
-	{
-		return; // whole block
-	}
-	for (int k = int(threadIdx.x); k < kFilterTileW * kFilterTileH; k += 128)
-	{
-		const int x = firstX + (k % kFilterTileW - 2) * step;
-		const int y = firstY + (k / kFilterTileW - 2) * step;
-		FilterTexel t = { outsideTexel(), make_float4(0.0f, 0.0f, 0.0f, 0.0f) };
-		if (x >= 0 && x < w && y >= 0 && y < h)
-		{
-			const V4 color = loadH4(input, y * w + x);
-			t.geometry = geometryTexel(receiver, normal, y * w + x, luminance(color.xyz()));
-			t.color = make_float4(color.x, color.y, color.z, color.w);
-		}
-		tile[k] = t;
-	}
-	__syncthreads();
-	const int lx = int(threadIdx.x) % kFilterW, ly = int(threadIdx.x) / kFilterW;
-	const int px = firstX + lx * step, py = firstY + ly * step;
-	if (px >= w || py >= h)
-	{
-		return;
-	}
 	const int i = py * w + px;
-	const int center = (ly + 2) * kFilterTileW + lx + 2;
-	const float4 n4 = tile[center].geometry.normal;
+	const float4 n4 = center.normal;
 	if (n4.w < 0.5f)
 	{
 		storeH4(out, i, v4(0.0f, 0.0f, 0.0f, 0.0f));
 		return;
 	}
 	const V3 n = v3(n4.x, n4.y, n4.z);
-	const float4 p4 = tile[center].geometry.position;
+	const float4 p4 = center.position;
 	const V3 position = v3(p4.x, p4.y, p4.z);
 	const float centerLuminance = p4.w;
 	float variance = 0.0f;
@@ -237,7 +214,7 @@ __global__ void __launch_bounds__(128) atrousKernel(const RestirParams P, int st
 #pragma unroll
 		for (int x = -2; x <= 2; ++x)
 		{
-			const FilterTexel& t = tile[center + y * kFilterTileW + x];
+			const FilterTexel& t = tap(x, y);
 			const float4 tn = t.geometry.normal;
 			if (tn.w < 0.0f)
 			{
@@ -257,6 +234,62 @@ __global__ void __launch_bounds__(128) atrousKernel(const RestirParams P, int st
 		}
 	}
 	storeH4(out, i, v4(colorSum / weightSum, varianceSum / (weightSum * weightSum)));
+}
+
+// One a-trous level. A pixel's taps lie step texels apart, so the pixels of one
+// residue (x mod step, y mod step) filter among themselves: a block takes 16x8
+// of them and its 20x12 texels go to shared memory once, the
+// normals normalised there. Every tap used to fetch 40 bytes and normalise the
+// neighbour's normal (a square root and a division, 24 times per texel instead
+// of 1.9) at 220 instructions a tap. Bound by issue (79% of the slots busy);
+// five levels at 960x540 take 0.36 ms, before 0.52 ms; the rows are a loop, so
+// that its 1,360 instructions stay in the instruction cache (unrolled: 0.42 ms).
+constexpr int kFilterTileW = kFilterW + 4, kFilterTileH = kFilterH + 4;
+
+__global__ void __launch_bounds__(128) atrousKernel(const RestirParams P, int step, int residuesX, int residuesY,
+	int blocksX, const uint16_t* __restrict__ input, const float4* __restrict__ receiver, const float4* __restrict__ normal, uint16_t* out)
+{
+	__shared__ FilterTexel tile[kFilterTileW * kFilterTileH];
+	const int w = int(P.gi_width), h = int(P.gi_height);
+	// Neighbouring blocks take neighbouring residues: they read the same lines.
+	const int blockX = int(blockIdx.x % uint32_t(blocksX)), blockY = int(blockIdx.x / uint32_t(blocksX));
+	const int firstX = blockX % residuesX + blockX / residuesX * kFilterW * step;
+	const int firstY = blockY % residuesY + blockY / residuesY * kFilterH * step;
+	if (firstX >= w || firstY >= h)
+	{
+		return; // whole block
+	}
+	for (int k = int(threadIdx.x); k < kFilterTileW * kFilterTileH; k += 128)
+	{
+		tile[k] = filterTexel(input, receiver, normal, w, h, firstX + (k % kFilterTileW - 2) * step,
+			firstY + (k / kFilterTileW - 2) * step);
+	}
+	__syncthreads();
+	const int lx = int(threadIdx.x) % kFilterW, ly = int(threadIdx.x) / kFilterW;
+	const int px = firstX + lx * step, py = firstY + ly * step;
+	if (px >= w || py >= h)
+	{
+		return;
+	}
+	const int center = (ly + 2) * kFilterTileW + lx + 2;
+	filterPixel(P, input, out, px, py, tile[center].geometry,
+		[&](int x, int y) -> const FilterTexel& { return tile[center + y * kFilterTileW + x]; });
+}
+
+// The same with the taps read from the image: for steps so large that a
+// residue's pixels leave most of a tile empty (restir_svgf_atrous).
+__global__ void __launch_bounds__(128) atrousDirectKernel(const RestirParams P, int step, const uint16_t* __restrict__ input,
+	const float4* __restrict__ receiver, const float4* __restrict__ normal, uint16_t* out)
+{
+	const int w = int(P.gi_width), h = int(P.gi_height);
+	const int px = int(blockIdx.x) * kFilterW + int(threadIdx.x) % kFilterW;
+	const int py = int(blockIdx.y) * kFilterH + int(threadIdx.x) / kFilterW;
+	if (px >= w || py >= h)
+	{
+		return;
+	}
+	filterPixel(P, input, out, px, py, filterTexel(input, receiver, normal, w, h, px, py).geometry,
+		[&](int x, int y) { return filterTexel(input, receiver, normal, w, h, px + x * step, py + y * step); });
 }
 
 // The split-sum specular albedo, brdf.sh:68-76 (Karis' analytic fit).
@@ -426,8 +459,27 @@ extern "C" int restir_svgf_atrous(const RestirParams* params, int step, const ui
 	const uint32_t residuesX = min(s, params->gi_width), residuesY = min(s, params->gi_height);
 	const uint32_t blocksX = ((params->gi_width + s - 1u) / s + kFilterW - 1u) / kFilterW * residuesX;
 	const uint32_t blocksY = ((params->gi_height + s - 1u) / s + kFilterH - 1u) / kFilterH * residuesY;
-	atrousKernel<<<blocksX * blocksY, 128, 0, asStream(stream)>>>(*params, int(s), int(residuesX), int(residuesY), int(blocksX),
-		input, reinterpret_cast<const float4*>(receiver), reinterpret_cast<const float4*>(normal), output);
+	// Tiles where the residues fill them well, or all blocks are in flight at once;
+	// the farther the taps, the more of them lie outside the image, which a tile
+	// does not gain from. us, tiles / taps from the image: 1920x1080, step 16 (88%
+	// full) 283 / 324, 40 (84%) 274 / 320, 48 (78%) 311 / 311, 80 (63%) 348 / 298,
+	// 96 (44%) 449 / 291, 256 (25%) 576 / 236; 960x540, 16 (79%) 84 / 92, 32 (66%)
+	// 86 / 86, 48 (44%) 125 / 84; 640x360, 48 (78%) 49 / 41; 128x128, 28 (16%, 784
+	// blocks) 18 / 23, 40 (8%, 1,600 blocks) 25 / 18.
+	const uint64_t tilePixels = uint64_t(blocksX) * blocksY * (kFilterW * kFilterH);
+	const uint64_t pixels = uint64_t(params->gi_width) * params->gi_height;
+	const cudaStream_t queue = asStream(stream);
+	if ((s < 48u && pixels * 10u >= tilePixels * 7u) || uint64_t(blocksX) * blocksY <= 148u * 8u)
+	{
+		atrousKernel<<<blocksX * blocksY, 128, 0, queue>>>(*params, int(s), int(residuesX), int(residuesY), int(blocksX),
+			input, reinterpret_cast<const float4*>(receiver), reinterpret_cast<const float4*>(normal), output);
+	}
+	else
+	{
+		const dim3 grid((params->gi_width + kFilterW - 1) / kFilterW, (params->gi_height + kFilterH - 1) / kFilterH);
+		atrousDirectKernel<<<grid, 128, 0, queue>>>(*params, int(s), input, reinterpret_cast<const float4*>(receiver),
+			reinterpret_cast<const float4*>(normal), output);
+	}
 	return launchStatus();
 }
 

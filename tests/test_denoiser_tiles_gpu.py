@@ -48,3 +48,24 @@ def test_tiles(size):
         rb.check(rb.load().restir_svgf_atrous(params, step, got.data_ptr(), receiver, normal, out.data_ptr(), None), "atrous")
         torch.cuda.synchronize()
         np.testing.assert_array_equal(out.cpu().numpy(), filtered, err_msg=str(step))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("size", [(320, 180), (641, 359)])
+def test_taps_from_the_image(size):
+    """Steps on both sides of the line between tiles and taps read from the image (as many blocks as are in flight at
+    once, tiles mostly empty), up to the image's size."""
+    import torch
+    w, h = size
+    color, moments, receiver, normal = inputs(w, h, seed=h)
+    params = RestirParams()
+    params.gi_width, params.gi_height, params.scene_scale = w, h, 0.7
+    source, positions, normals = (torch.from_numpy(a).cuda() for a in (color, receiver, normal))
+    for step in (16, 32, 33, 47, 48, 100, w - 1, w, w + 1):
+        want = np.zeros_like(color)
+        out = torch.zeros_like(source)
+        ob.load().oracle_svgf_atrous(params, step, color.ctypes.data, receiver.ctypes.data, normal.ctypes.data, want.ctypes.data)
+        rb.check(rb.load().restir_svgf_atrous(params, step, source.data_ptr(), positions.data_ptr(), normals.data_ptr(),
+                                              out.data_ptr(), None), "atrous")
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(out.cpu().numpy(), want, err_msg=str(step))
