@@ -10,9 +10,11 @@
 // entries (each lane carries the larger value onwards), which leaves the
 // same list whatever the arrival order. Bound by the latency of the atomics
 // of one lane, up to C in a row; the cascade starts behind the entries known
-// to be smaller (below): 0.172 -> 0.055 ms alone for the 960x540 receivers of
-// the 1M-triangle city, C 32; with as good as all blocks in flight at once
-// (256x256) there is little to skip, 0.016 and 0.018 ms.
+// to be smaller (below). us after the clear, from slot 0 / behind an entry
+// found by halves / by quarters, C 32: 960x540 receivers of the 1M-triangle city
+// 231 / 58 / 56, 256x256 30.7 / 23.3 / 22.6, 128x128 of the courtyard 20.5 / 22.6
+// / 21.5; where all blocks are in flight at once and cells are large there is
+// little to skip: 256x256 of the Cornell box 16.4 / 18.4 / 18.4.
 #include "grid.cuh"
 #include "screen.cuh"
 
@@ -42,6 +44,7 @@ __global__ void __launch_bounds__(256) gridClearKernel(uint4* counts, uint32_t c
 	}
 }
 
+template<bool kOrdered>
 __global__ void __launch_bounds__(256) gridInsertKernel(const RestirParams P, const float* __restrict__ depth,
 	const uint8_t* __restrict__ normal, uint32_t* grid)
 {
@@ -112,32 +115,48 @@ __global__ void __launch_bounds__(256) gridInsertKernel(const RestirParams P, co
 	// list, or a full one. The r-th peer has r smaller ones beside it and starts
 	// r slots later.
 	uint32_t start = 0u;
-	if (P.grid_mode == RESTIR_GRID_DETERMINISTIC && claimed != kGridInvalid)
+	if (kOrdered && claimed != kGridInvalid)
 	{
 		const uint32_t* cell = grid + 2u * T + claimed * C;
 		uint32_t end = base < C ? base : C;
 		while (start < end)
 		{
-			const uint32_t middle = (start + end) / 2u;
-			if (__ldcg(cell + middle) < uint32_t(i))
+			// Three entries a round: a round is one latency.
+			const uint32_t first = start, count = end - start;
+			uint32_t entry[3];
+#pragma unroll
+			for (uint32_t q = 0u; q < 3u; ++q)
 			{
-				start = middle + 1u;
+				entry[q] = __ldcg(cell + first + count * (q + 1u) / 4u);
 			}
-			else
+#pragma unroll
+			for (uint32_t q = 0u; q < 3u; ++q)
 			{
-				end = middle;
+				const uint32_t at = first + count * (q + 1u) / 4u;
+				if (entry[q] < uint32_t(i))
+				{
+					start = at + 1u;
+				}
+				else
+				{
+					end = min(end, at);
+				}
 			}
+			start = min(start, end); // entries out of order, still on their way: the lower start holds too
 		}
 	}
 	claimed = __shfl_sync(0xffffffffu, claimed, leader);
 	base = __shfl_sync(0xffffffffu, base, leader);
-	start = __shfl_sync(0xffffffffu, start, leader);
+	if (kOrdered)
+	{
+		start = __shfl_sync(0xffffffffu, start, leader);
+	}
 	if (!active || claimed == kGridInvalid)
 	{
 		return;
 	}
 	uint32_t* entries = grid + 2u * T + claimed * C;
-	if (P.grid_mode == RESTIR_GRID_DETERMINISTIC)
+	if (kOrdered)
 	{
 		uint32_t value = uint32_t(i);
 		for (uint32_t k = start + rank; k < C && value != kGridInvalid; ++k)
@@ -191,7 +210,9 @@ extern "C" int restir_grid_insert(const RestirParams* params, const RestirGBuffe
 		return RESTIR_ERROR_INVALID_ARGUMENT;
 	}
 	const uint32_t pixels = params->gi_width * params->gi_height;
-	gridInsertKernel<<<(pixels + 255u) / 256u, 256, 0, asStream(stream)>>>(*params, gbuffer->depth, gbuffer->normal, grid);
+	const bool ordered = params->grid_mode == RESTIR_GRID_DETERMINISTIC;
+	(ordered ? gridInsertKernel<true> : gridInsertKernel<false>)<<<(pixels + 255u) / 256u, 256, 0, asStream(stream)>>>(*params,
+		gbuffer->depth, gbuffer->normal, grid);
 	return launchStatus();
 }
 
