@@ -304,12 +304,14 @@ __device__ __forceinline__ V3 compositeSpecularAlbedo(V3 f0, float roughness, fl
 
 // fs_composite.sc:48-143 with the final view's options; the indirect
 // specular when a specular target is given.
-// Bound by the latency of its taps and divisions: eight blocks a SM (64
-// registers, 40 bytes spilled) where 94 registers left five: 0.201 -> 0.145 ms
-// at 1920x1080, 0.094 -> 0.073 ms at 1280x720, 0.0116 -> 0.0125 at 256x256, where
-// three and a half blocks a SM are all there are; ten blocks gain 0.007 ms more
-// there and lose 0.002 here.
-__global__ void __launch_bounds__(128, 8) compositeKernel(const RestirParams P, RestirGBuffer gb, const float* __restrict__ atlas,
+// Bound by the latency of its taps and divisions. kBlocks: blocks a SM; eight
+// (64 registers, 40 bytes spilled) where 94 registers left five: 189 -> 144 us
+// at 1920x1080 (courtyard), 75 -> 62 at 1280x720, 19 -> 15 at 480x270. Images of
+// no more than five blocks a SM run in one wave either way and take the
+// registers: 320x180 12.5 -> 10.6 (Cornell box), 256x256 with the specular target
+// 14.5 -> 12.5.
+template<int kBlocks>
+__global__ void __launch_bounds__(128, kBlocks) compositeKernel(const RestirParams P, RestirGBuffer gb, const float* __restrict__ atlas,
 	const uint16_t* __restrict__ gi, const uint16_t* __restrict__ diDiffuse, const uint16_t* __restrict__ diSpecular,
 	const uint16_t* __restrict__ specularTarget, uint16_t* hdr)
 {
@@ -426,6 +428,16 @@ __global__ void __launch_bounds__(128, 8) compositeKernel(const RestirParams P, 
 	storeH4(hdr, i, v4(result, 1.0f));
 }
 
+int launchComposite(const RestirParams& params, const RestirGBuffer& gbuffer, const float* shadowAtlas, const uint16_t* gi,
+	const uint16_t* diDiffuse, const uint16_t* diSpecular, const uint16_t* specular, uint16_t* hdr, cudaStream_t s)
+{
+	const dim3 grid((params.width + 15) / 16, (params.height + 7) / 8);
+	const bool oneWave = uint64_t(grid.x) * grid.y <= 148u * 5u;
+	(oneWave ? compositeKernel<5> : compositeKernel<8>)<<<grid, 128, 0, s>>>(params, gbuffer, shadowAtlas, gi, diDiffuse, diSpecular,
+		specular, hdr);
+	return launchStatus();
+}
+
 } // namespace
 } // namespace restir
 
@@ -492,10 +504,7 @@ extern "C" int restir_composite(const RestirParams* params, const RestirGBuffer*
 	{
 		return RESTIR_ERROR_INVALID_ARGUMENT;
 	}
-	dim3 grid((params->width + 15) / 16, (params->height + 7) / 8);
-	compositeKernel<<<grid, 128, 0, asStream(stream)>>>(*params, *gbuffer, shadow_atlas, gi, di_diffuse, di_specular, nullptr,
-		hdr);
-	return launchStatus();
+	return launchComposite(*params, *gbuffer, shadow_atlas, gi, di_diffuse, di_specular, nullptr, hdr, asStream(stream));
 }
 
 extern "C" int restir_composite_specular(const RestirParams* params, const RestirGBuffer* gbuffer, const float* shadow_atlas,
@@ -508,8 +517,5 @@ extern "C" int restir_composite_specular(const RestirParams* params, const Resti
 	{
 		return RESTIR_ERROR_INVALID_ARGUMENT;
 	}
-	dim3 grid((params->width + 15) / 16, (params->height + 7) / 8);
-	compositeKernel<<<grid, 128, 0, asStream(stream)>>>(*params, *gbuffer, shadow_atlas, gi, di_diffuse, di_specular, specular,
-		hdr);
-	return launchStatus();
+	return launchComposite(*params, *gbuffer, shadow_atlas, gi, di_diffuse, di_specular, specular, hdr, asStream(stream));
 }
