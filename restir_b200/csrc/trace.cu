@@ -249,7 +249,8 @@ extern "C" int restir_trace(const RestirParams* params, const RestirScene* scene
 	{
 		launchThreads<RESTIR_TRACE_CLOSEST>(bvh, arrays, n, s);
 	}
-	else if (kind == RESTIR_TRACE_CLOSEST_STACKLESS && n > kFourLaneRays && n <= 2u * kResidentLanes)
+	else if ((kind == RESTIR_TRACE_CLOSEST_STACKLESS && n > kFourLaneRays && n <= 2u * kResidentLanes)
+		|| (bvh.nodeCount == 0 && kind != RESTIR_TRACE_CLOSEST_QUEUE)) // nothing to hit, and no ray to count
 	{
 		launchThreads<RESTIR_TRACE_CLOSEST_STACKLESS>(bvh, arrays, n, s);
 	}

@@ -165,3 +165,24 @@ def test_nearest_hits_on_both_sides_of_each_line(triangles, n):
         > {6_000: 0, 30_000: 12_288, 100_000: 131_072}[triangles]
     check(setup, seeded_rays(setup, n, seed=11), rb.TRACE_CLOSEST)
     check(setup, seeded_rays(setup, n - 1, seed=12), rb.TRACE_CLOSEST)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind, counted", [(rb.TRACE_CLOSEST, 0), (rb.TRACE_ANY, 0), (rb.TRACE_CLOSEST_STACKLESS, 0),
+                                           (rb.TRACE_ANY_WAVE, 0), (rb.TRACE_CLOSEST_QUEUE, 1)])
+@pytest.mark.parametrize("n", [40, 40_000, 400_000])
+def test_empty_scene(kind, counted, n):
+    """Rays in a scene without nodes hit nothing, and only the queue's kind counts them."""
+    import ctypes as C
+    import torch
+    scene = make_scene(rb.SCENE_CORNELL).device_scene()
+    scene.node_count = 0
+    rays = torch.ones((n, 8), dtype=torch.float32, device="cuda")
+    ids, t = torch.zeros(n, dtype=torch.int32, device="cuda"), torch.zeros(n, dtype=torch.float32, device="cuda")
+    values = (C.c_uint64 * 8)()
+    rb.check(rb.load().restir_counters(1, values), "counters")
+    rb.check(rb.load().restir_trace(None, scene, rays.data_ptr(), ids.data_ptr(), t.data_ptr(), n, kind, None), "restir_trace")
+    torch.cuda.synchronize()
+    rb.check(rb.load().restir_counters(0, values), "counters")
+    assert (ids == -1).all() and (t == 1.0).all()
+    assert sum(values[0:4]) == counted * n
