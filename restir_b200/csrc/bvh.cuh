@@ -582,9 +582,9 @@ __device__ __forceinline__ int nearestFirstLoop(const BvhView& b, const SlabRay&
 
 // kSplit: the rays of a tile nearly always agree on the signs of their
 // directions: a copy of the loop for each combination, and one for warps that
-// disagree (G-buffer of the 1080p city frame 0.50 -> 0.43 ms, shadow atlas 0.97
-// -> 0.89 ms with the words carried; the loop was bound by the ALU pipe, 69%
-// busy, on which minima and maxima run).
+// disagree (G-buffer of the 1080p city frame 0.50 -> 0.43 ms with the words
+// carried; the loop was bound by the ALU pipe, 69% busy, on which minima and
+// maxima run).
 template<bool kWide, bool kSplit, bool kConservative, typename Test, typename Accept>
 __device__ inline int traceNearestFirst(const BvhView& b, V3 o, V3 d, float& distance, Test test, Accept accept)
 {

@@ -21,7 +21,7 @@ namespace restir
 namespace
 {
 
-template<bool kWide, bool kSplit>
+template<bool kWide>
 __global__ void __launch_bounds__(64) gbufferKernel(const RestirParams P, BvhView bvh, const float4* __restrict__ normals,
 	const float4* __restrict__ materials, RestirGBuffer gb)
 {
@@ -44,7 +44,7 @@ __global__ void __launch_bounds__(64) gbufferKernel(const RestirParams P, BvhVie
 	const float rayLength = length(span);
 	const V3 direction = span / rayLength;
 	float distance = rayLength;
-	const int hit = traceNearestFiltered<kWide, kSplit>(bvh, nearPoint, direction, distance, [&](int t)
+	const int hit = traceNearestFiltered<kWide, kWide>(bvh, nearPoint, direction, distance, [&](int t)
 	{
 		float4 n = __ldg(normals + t);
 		return n.w > 0.5f || dot(v3(n.x, n.y, n.z), camera - bvh.vertex(t, 0)) > 0.0f;
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(64) gbufferKernel(const RestirParams P, BvhVie
 	gb.depth[i] = clip.z / clip.w;
 }
 
-template<bool kWide, bool kSplit>
+template<bool kWide>
 __global__ void __launch_bounds__(64) shadowAtlasKernel(const RestirParams P, BvhView bvh, float* __restrict__ atlas)
 {
 	const int f = int(P.shadow_face_size);
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(64) shadowAtlasKernel(const RestirParams P, Bv
 	const float rayLength = length(span);
 	const V3 direction = span / rayLength;
 	float distance = rayLength;
-	const int hit = traceNearestFiltered<kWide, kSplit>(bvh, nearPoint, direction, distance, [](int) { return true; });
+	const int hit = traceNearestFiltered<kWide, false>(bvh, nearPoint, direction, distance, [](int) { return true; });
 	float value = 1.0f;
 	if (hit >= 0)
 	{
@@ -122,12 +122,6 @@ __global__ void __launch_bounds__(64) shadowAtlasKernel(const RestirParams P, Bv
 
 using namespace restir;
 
-// The instance for a scene: the loop is split by the directions' signs where
-// the rays visit enough nodes to pay for fetching the longer code (Cornell box
-// at 256x256: G-buffer 33 us, split 41 us; 4,096 nodes as in restir_trace).
-#define RESTIR_PICK_CAST(kernel, bvh) \
-	(!wideRows(bvh) ? kernel<false, false> : ((bvh).nodeCount > 4096 ? kernel<true, true> : kernel<true, false>))
-
 extern "C" int restir_gbuffer_primary(const RestirParams* params, const RestirScene* scene, const RestirGBuffer* gbuffer,
 	void* stream)
 {
@@ -139,7 +133,10 @@ extern "C" int restir_gbuffer_primary(const RestirParams* params, const RestirSc
 	}
 	dim3 grid((params->width + 7) / 8, (params->height + 7) / 8);
 	const BvhView bvh = makeBvhView(scene);
-	RESTIR_PICK_CAST(gbufferKernel, bvh)<<<grid, 64, 0, asStream(stream)>>>(*params, bvh,
+	// Split by the directions' signs (traceNearestFirst): us alone, split / not, at
+	// 1920x1080 in scenes of 43, 1,209, 10k and 1.9M nodes 49 / 51, 185 / 202, 171 /
+	// 190, 433 / 482; at 256x256 27 / 28, 42 / 48, 54 / 60, 124 / 130.
+	(wideRows(bvh) ? gbufferKernel<true> : gbufferKernel<false>)<<<grid, 64, 0, asStream(stream)>>>(*params, bvh,
 		reinterpret_cast<const float4*>(scene->triangle_normals), reinterpret_cast<const float4*>(scene->materials), *gbuffer);
 	return launchStatus();
 }
@@ -153,6 +150,10 @@ extern "C" int restir_shadow_atlas(const RestirParams* params, const RestirScene
 	const uint32_t f = params->shadow_face_size;
 	dim3 grid((3 * f + 7) / 8, (2 * f + 7) / 8);
 	const BvhView bvh = makeBvhView(scene);
-	RESTIR_PICK_CAST(shadowAtlasKernel, bvh)<<<grid, 64, 0, asStream(stream)>>>(*params, bvh, atlas);
+	// Not split: alone its 512x512 faces gain little (10k nodes 122 us, split 126;
+	// 1.9M nodes 905 and 887), and in a frame, where it runs beside the other stream's
+	// passes, the longer code costs them: 1920x1080 in the 1M-triangle city 8.04 ms
+	// split, 7.98 not; 256x256 in the 100k-triangle city 2.29 and 2.18.
+	(wideRows(bvh) ? shadowAtlasKernel<true> : shadowAtlasKernel<false>)<<<grid, 64, 0, asStream(stream)>>>(*params, bvh, atlas);
 	return launchStatus();
 }
