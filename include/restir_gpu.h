@@ -429,7 +429,11 @@ int restir_counters(int enable, uint64_t* counters);
 
 /* Evaluates one numeric convention of restir_numeric.h on the device, for
  * tests: fn 0 sin, 1 cos, 2 exp, 3 half round trip (hardware), 4 half round
- * trip (restir_numeric.h), 5 unorm8 store, 6 floor(log2), 7 x^64. No
+ * trip (restir_numeric.h), 5 unorm8 store, 6 floor(log2), 7 x^64, 8 the
+ * generator's step, 9 the grid's checksum hash, 10 half to float, 11 log2, 12
+ * exp2, 13 x^2.2, 14 x^(1/2.2); the kernels' short forms, each beside what it
+ * stands for: 15, 16 x / 16.5, 17, 18 the byte of an AgX channel, 19, 20 of the
+ * other operators', 21, 22 a byte / 255. No
  * counterpart in the reference (a test hook). */
 int restir_numeric_eval(int fn, const float* input, float* output, uint32_t n, void* stream);
 

@@ -1,6 +1,8 @@
 // restir_numeric_eval: evaluates one function of include/restir_numeric.h
 // on the device over an array, so that tests can check that the kernels'
-// sin, cos, exp, half and unorm8 conversions are bit-identical to the host's.
+// sin, cos, exp, half and unorm8 conversions are bit-identical to the host's, and
+// that the kernels' short forms equal what they stand for.
+#include "display_bytes.cuh"
 #include "grid.cuh"
 
 namespace restir
@@ -34,6 +36,15 @@ __global__ void numericKernel(int fn, const float* __restrict__ in, float* __res
 	case 12: y = rn_exp2(x); break;
 	case 13: y = rn_pow(x, 2.2f); break;
 	case 14: y = rn_pow(x, 1.0f / 2.2f); break;
+	// The kernels' short forms, and what each stands for.
+	case 15: y = agxShare(x); break;
+	case 16: y = x / 16.5f; break;
+	case 17: y = float(gammaByte(x, true)); break;
+	case 18: y = float(gammaByteExact(x, true)); break;
+	case 19: y = float(gammaByte(x, false)); break;
+	case 20: y = float(gammaByteExact(x, false)); break;
+	case 21: y = unorm8(uint32_t(x)); break;
+	case 22: y = x / 255.0f; break;
 	default: y = x; break;
 	}
 	out[i] = y;

@@ -1,5 +1,8 @@
 """The ABI's numeric conventions (include/restir_numeric.h): accuracy of the
 host implementation against numpy, and bit-identity of the device's."""
+import re
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -119,3 +122,74 @@ def test_unorm8_two_term_product():
     # u * head (at most 32 bits) plus the small term is exact in binary64: rounding it to float is the fused operation.
     fused = (u.astype(np.float64) * np.float64(head) + np.float64(u * tail)).astype(np.float32)
     np.testing.assert_array_equal(fused, u / np.float32(255.0))
+
+
+def scaled_by_products(x, exponent):
+    """p * 2^n1 * 2^n2 with n1 + n2 = exponent, the two exact steps of restir_numeric.h's exponentials."""
+    half = (exponent / 2).astype(np.int32)  # towards zero
+    scale = [np.ldexp(np.float32(1.0), n).astype(np.float32) for n in (half, exponent - half)]
+    return (x * scale[0]) * scale[1]
+
+
+def test_exponentials_by_exponent_and_by_products():
+    """rn_exp between -86 and 86 and rn_exp2 between -120 and 120 add to the exponent where the general form multiplies
+    twice: the same on every 101st float of their range and all those next to its ends."""
+    one = np.float32(1.0)
+
+    def floats(end):
+        top = int(np.array([end], np.float32).view(np.int32)[0])
+        bits = np.concatenate([np.arange(0, top, 101), np.arange(top - 5000, top + 5000)]).astype(np.int32)
+        x = bits.view(np.float32)
+        return np.concatenate([x, -x])
+
+    def rounded(x):
+        i = (np.abs(x) + np.float32(0.5)).astype(np.int32)
+        return np.where(x < 0, -i, i).astype(np.int32)
+
+    def series(r):
+        p = np.full_like(r, np.float32(2.4801587301587302e-05))
+        for c in (1.98412698412698413e-04, 1.38888888888888889e-03, 8.33333333333333333e-03, 4.16666666666666667e-02,
+                  1.66666666666666667e-01, 0.5):
+            p = p * r + np.float32(c)
+        return (p * r + one) * r + one
+
+    header = (Path(__file__).resolve().parent.parent / "include" / "restir_numeric.h").read_text()
+    constant = {n: np.float32(re.search(rf"#define RN_{n} ([^\s]+?)f?\s", header).group(1))
+                for n in ("LOG2E", "LN2_HI", "LN2_LO", "LN2")}
+    x = floats(86.0)
+    n = rounded(x * constant["LOG2E"])
+    k = n.astype(np.float32)
+    r = (x - k * constant["LN2_HI"]) - k * constant["LN2_LO"]
+    np.testing.assert_array_equal(host_eval(2, x).view(np.uint32), scaled_by_products(series(r), n).view(np.uint32))
+    x = floats(120.0)
+    n = rounded(x)
+    p = host_eval(2, (x - n.astype(np.float32)) * constant["LN2"])
+    np.testing.assert_array_equal(host_eval(12, x).view(np.uint32), scaled_by_products(p, n).view(np.uint32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("short, whole, first, last", [
+    (17, 18, 0.0, 1.0),                      # AgX clamps its channels to [0, 1]
+    (19, 20, 0.0, np.inf), (19, 20, -0.0, -np.inf),
+    (15, 16, 4e-37, 17.0),                   # AgX's stops above the darkest
+    (21, 22, None, None)])
+def test_short_forms_equal_what_they_stand_for(short, whole, first, last):
+    """Every float of each range on the device, and NaN for the bytes."""
+    import torch
+
+    def same(x):
+        out = [torch.empty_like(x) for _ in range(2)]
+        for fn, y in zip((short, whole), out):
+            rb.check(rb.load().restir_numeric_eval(fn, x.data_ptr(), y.data_ptr(), x.numel(), None), "numeric")
+        return torch.equal(out[0].view(torch.int32), out[1].view(torch.int32))
+
+    if first is None:
+        assert same(torch.arange(256, dtype=torch.float32, device="cuda"))
+        return
+    low, high = (int(np.array([v], np.float32).view(np.uint32)[0]) for v in (first, last))
+    step = 1 << 26
+    for start in range(low, high + 1, step):
+        bits = torch.arange(start, min(start + step, high + 1), dtype=torch.int64, device="cuda")
+        assert same(torch.where(bits > 0x7fffffff, bits - (1 << 32), bits).to(torch.int32).view(torch.float32)), hex(start)
+    if whole != 16:
+        assert same(torch.full((4,), torch.nan, device="cuda"))
