@@ -186,3 +186,41 @@ def test_empty_scene(kind, counted, n):
     rb.check(rb.load().restir_counters(0, values), "counters")
     assert (ids == -1).all() and (t == 1.0).all()
     assert sum(values[0:4]) == counted * n
+
+
+class Shifted(SceneSetup):
+    """A scene whose device rows start 16 bytes past a 32-byte boundary."""
+
+    def device_scene(self):
+        import torch
+        scene = super().device_scene()
+        data = self.bvh_data if self.bvh_data is not None else self.bvh.data
+        rows = torch.zeros(data.size + 4, dtype=torch.float32, device="cuda")
+        rows[4:] = torch.from_numpy(data).cuda()
+        self.keep.append(rows)
+        scene.bvh = rows[4:].data_ptr()
+        return scene
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("wavefront", [False, True])
+@pytest.mark.parametrize("rows", ["shifted", "padded"])
+def test_frame_of_rows_on_16_bytes(rows, wavefront):
+    """Every pass that traces, through its instance for rows that cannot be read 32 bytes at a time: a buffer on 16
+    bytes, and one row of padding before the triangles."""
+    from oracle.frame import run_checked
+    setup = make_scene(rb.SCENE_COURTYARD, 3, 20_000, extra_lights=8)
+    if rows == "padded":
+        padded(setup, 1)
+    else:
+        setup = Shifted(setup.mesh, setup.bvh, setup.lights, setup.settings, setup.materials)
+    assert not rb.load().restir_bvh_wide_rows(setup.device_scene())
+    setup.settings.grid_mode = rb.GRID_DETERMINISTIC
+    report, _, _ = run_checked(setup, 112, 62, 3, setup.settings, gi_wavefront=wavefront)
+    assert report == {}, report
+
+
+@pytest.mark.gpu
+def test_watertight_unaligned_rows():
+    setup = make_scene(rb.SCENE_CITY, 0, 60_000)
+    check(setup, seeded_rays(setup, 20_000, seed=8), rb.TRACE_CLOSEST_WATERTIGHT, offset=4)
