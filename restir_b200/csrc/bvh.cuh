@@ -217,11 +217,14 @@ __device__ inline int traceStacklessWave(const BvhView& b, V3 o, V3 d, bool anyH
 	return hit;
 }
 
-// bvh.sh:216-295. stack: this thread's kBvhShortStack entries, stride apart
-// (shared memory, interleaved across the block's threads).
-__device__ inline int traceShortStack(const BvhView& b, V3 o, V3 d, float& distance, int* stack, int stride, TraceWork& work)
+// The nearest-first walk of bvh.sh:216-295 up to its re-walk, which is to follow
+// when dropped. stack: this thread's kBvhShortStack entries, stride apart (shared
+// memory, interleaved across the block's threads).
+__device__ __forceinline__ int walkShortStack(const BvhView& b, V3 o, V3 d, float& distance, int* stack, int stride,
+	TraceWork& work, bool& dropped)
 {
 	V3 inv = bvhInverseDirection(d);
+	dropped = false;
 	++work.nodes;
 	if (intersectBox(o, inv, b.row(0).xyz(), b.row(1).xyz(), distance) < 0.0f)
 	{
@@ -229,7 +232,6 @@ __device__ inline int traceShortStack(const BvhView& b, V3 o, V3 d, float& dista
 	}
 	int stackTop = 0;
 	int stackCount = 0;
-	bool dropped = false;
 	int hit = -1;
 	int node = 0;
 	int step = 0;
@@ -284,6 +286,14 @@ __device__ inline int traceShortStack(const BvhView& b, V3 o, V3 d, float& dista
 	{
 		reportTruncatedRay();
 	}
+	return hit;
+}
+
+// bvh.sh:216-295.
+__device__ inline int traceShortStack(const BvhView& b, V3 o, V3 d, float& distance, int* stack, int stride, TraceWork& work)
+{
+	bool dropped;
+	int hit = walkShortStack(b, o, d, distance, stack, stride, work, dropped);
 	if (dropped)
 	{
 		int stacklessHit = traceStacklessWalk(b, o, d, false, distance, work);

@@ -24,27 +24,46 @@ constexpr int kTraceBlock = 128;
 //   stackless, city of 47k nodes, 64,000: 4 158, 1 148, w 156; 200,000: 4 293,
 //     1 251, w 263; of 1.9M, 1,000,000: 1 3,762, w 2,502; Cornell box, 300,000:
 //     1 49, w 56; 500,000: 1 73, w 73;
-//   closest, city of 1.9M nodes, 1: 1 70, w 89; 1,000: 1 268, w 225; 1,000,000:
-//     1 2,325, w 1,813; of 190k, 32: 1 101, w 115; 200: 1 107, w 118; 200,000:
-//     1 396, w 410; of 47k, 16,000: 1 60, w 74; 300,000: 1 159, w 180; 500,000:
-//     1 216, w 215; of 10k, 1,000,000: 1 220, w 228.
+//   closest (1r: one thread a ray, its re-walk by four lanes), city of 1.9M nodes,
+//     1: 1 70, w 89; 1,000: 1 268, w 225; 1,000,000: 1 2,325, w 1,813; of 190k, 32:
+//     1 101, w 115; 200,000: 1 396, w 410; of 47k, 16,000: 1 60, 1r 68, w 74;
+//     300,000: 1 159, 1r 175, w 180; 500,000: 1 216, w 215; courtyard of 40k nodes,
+//     16,000: 1 332, 1r 268, w 266; 300,000: 1 488, 1r 483, w 457; 1,000,000:
+//     Cornell box 1 134, w 157; 3.9k nodes 1 403, w 403; 10k (city) 1 220, w 228,
+//     (courtyard) 1 776, w 670.
 // So walks take four lanes up to a group of them for each ray that the SMs hold
 // at once (148 x 32 warps x 8), where they are latency-bound; then any hits take
 // the warp's shared leaves, stackless nearest hits one thread each until every
 // lane has two rays. Nearest hits take one thread each where a ray visits few
-// nodes or the rays are few: below 128, in scenes of up to 12,288 nodes always,
-// up to 131,072 nodes until every lane has three rays, and just past one ray a
-// lane, where the parts' last warps leave the SMs idle.
+// nodes or the rays are few (below 128, and in scenes of up to 4,096 nodes), and
+// past one ray a lane, where the parts' last warps leave the SMs idle; in scenes
+// of up to 131,072 nodes with a lane for every ray the four-lane re-walk is the
+// middle between the courtyard's long walks and the city's short ones.
 constexpr uint32_t kResidentLanes = 148u * 32u * 32u;
 constexpr uint32_t kFourLaneRays = kResidentLanes / 4u;
 constexpr uint32_t kFewRays = 128u;
-constexpr int kSmallScene = 12288;
+constexpr int kSmallScene = 4096;
 constexpr int kMiddleScene = 131072;
 
-bool nearestPerThread(uint32_t n, int nodes)
+enum class Nearest
 {
-	return n < kFewRays || nodes <= kSmallScene || (nodes <= kMiddleScene && n <= 3u * kResidentLanes)
-		|| (n > kResidentLanes && n <= kResidentLanes + kResidentLanes / 2u);
+	thread,
+	threadGroupRewalk,
+	part
+};
+
+Nearest nearestKernel(uint32_t n, int nodes)
+{
+	if (n < kFewRays || nodes <= kSmallScene)
+	{
+		return Nearest::thread;
+	}
+	if (nodes <= kMiddleScene && n <= kResidentLanes)
+	{
+		return Nearest::threadGroupRewalk;
+	}
+	const bool thread = n > kResidentLanes && n <= (nodes <= kMiddleScene ? 3u * kResidentLanes : kResidentLanes + kResidentLanes / 2u);
+	return thread ? Nearest::thread : Nearest::part;
 }
 
 // A contiguous part of the ray set, one per warp: its lanes take the part's
@@ -93,6 +112,38 @@ __global__ void __launch_bounds__(kTraceBlock, 8) nearestPartsKernel(BvhView bvh
 	traceNearest<kWide>(bvh, source, storage[threadIdx.x >> 5]);
 	__syncwarp(); // the warp's stores
 	MarkedSource<4> marked{ arrays, first, end, nullptr };
+	traceGroupWalks<false, kWide>(bvh, marked);
+}
+
+// One thread per ray, and the rays whose short stack dropped entries by four
+// lanes each afterwards: the re-walk is the longest part of such a ray, and in
+// one thread it holds up its warp.
+template<bool kWide>
+__global__ void __launch_bounds__(kTraceBlock) nearestThreadsKernel(BvhView bvh, RayArrays arrays, uint32_t n)
+{
+	__shared__ int stack[kBvhShortStack * kTraceBlock];
+	const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+	const uint32_t first = i & ~31u;
+	if (first >= n)
+	{
+		return; // whole warp
+	}
+	if (i < n)
+	{
+		Ray r;
+		arrays.load(i, r);
+		if (bvh.available())
+		{
+			TraceWork work;
+			bool dropped;
+			r.hit = walkShortStack(bvh, r.o, r.d, r.distance, stack + threadIdx.x, kTraceBlock, work, dropped);
+			countWork(RESTIR_COUNT_CLOSEST, work.nodes, work.triangles);
+			r.hit = dropped ? markedHit(r.hit) : r.hit;
+		}
+		arrays.store(r);
+	}
+	__syncwarp(); // the warp's stores
+	MarkedSource<4> marked{ arrays, first, n - first > 32u ? first + 32u : n, nullptr };
 	traceGroupWalks<false, kWide>(bvh, marked);
 }
 
@@ -150,11 +201,15 @@ __global__ void __launch_bounds__(kTraceBlock) traceKernel(BvhView bvh, RayArray
 	arrays.store(r);
 }
 
+uint32_t threadBlocks(uint32_t n)
+{
+	return uint32_t((uint64_t(n) + kTraceBlock - 1) / kTraceBlock);
+}
+
 template<int kKind, bool kWide = false>
 void launchThreads(const BvhView& bvh, const RayArrays& arrays, uint32_t n, cudaStream_t s)
 {
-	const uint32_t blocks = uint32_t((uint64_t(n) + kTraceBlock - 1) / kTraceBlock);
-	traceKernel<kKind, kWide><<<blocks, kTraceBlock, 0, s>>>(bvh, arrays, n);
+	traceKernel<kKind, kWide><<<threadBlocks(n), kTraceBlock, 0, s>>>(bvh, arrays, n);
 }
 
 // Rays per warp: as few as fill the SMs once (148 x 32 warps resident), a
@@ -230,6 +285,7 @@ extern "C" int restir_trace(const RestirParams* params, const RestirScene* scene
 	BvhView bvh = makeBvhView(scene);
 	cudaStream_t s = asStream(stream);
 	const RayArrays arrays = { reinterpret_cast<const float4*>(rays), hit_triangle, hit_distance };
+	const Nearest nearest = nearestKernel(n, bvh.nodeCount);
 	if (kind == RESTIR_TRACE_ANY_WAVE)
 	{
 		launchThreads<RESTIR_TRACE_ANY_WAVE>(bvh, arrays, n, s);
@@ -245,9 +301,13 @@ extern "C" int restir_trace(const RestirParams* params, const RestirScene* scene
 			launchThreads<RESTIR_TRACE_CLOSEST_WATERTIGHT>(bvh, arrays, n, s);
 		}
 	}
-	else if (kind == RESTIR_TRACE_CLOSEST && nearestPerThread(n, bvh.nodeCount))
+	else if (kind == RESTIR_TRACE_CLOSEST && nearest == Nearest::thread)
 	{
 		launchThreads<RESTIR_TRACE_CLOSEST>(bvh, arrays, n, s);
+	}
+	else if (kind == RESTIR_TRACE_CLOSEST && nearest == Nearest::threadGroupRewalk)
+	{
+		(wideRows(bvh) ? nearestThreadsKernel<true> : nearestThreadsKernel<false>)<<<threadBlocks(n), kTraceBlock, 0, s>>>(bvh, arrays, n);
 	}
 	else if ((kind == RESTIR_TRACE_CLOSEST_STACKLESS && n > kFourLaneRays && n <= 2u * kResidentLanes)
 		|| (bvh.nodeCount == 0 && kind != RESTIR_TRACE_CLOSEST_QUEUE)) // nothing to hit, and no ray to count

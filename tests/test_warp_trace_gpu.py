@@ -156,13 +156,13 @@ def test_more_than_2_31_rays():
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("triangles", [6_000, 30_000, 100_000])
+@pytest.mark.parametrize("triangles", [2_000, 30_000, 100_000])
 @pytest.mark.parametrize("n", [127, 128, 151_553, 227_329, 454_657])
 def test_nearest_hits_on_both_sides_of_each_line(triangles, n):
     """The sizes of scene and ray set between which restir_trace changes its kernel for nearest hits."""
     setup = make_scene(rb.SCENE_CITY, 0, triangles)
-    assert {6_000: 12_288, 30_000: 131_072, 100_000: 1 << 30}[triangles] > setup.bvh.desc.node_count \
-        > {6_000: 0, 30_000: 12_288, 100_000: 131_072}[triangles]
+    assert {2_000: 4_096, 30_000: 131_072, 100_000: 1 << 30}[triangles] > setup.bvh.desc.node_count \
+        > {2_000: 0, 30_000: 4_096, 100_000: 131_072}[triangles]
     check(setup, seeded_rays(setup, n, seed=11), rb.TRACE_CLOSEST)
     check(setup, seeded_rays(setup, n - 1, seed=12), rb.TRACE_CLOSEST)
 
