@@ -151,7 +151,7 @@ struct MarkedSource
 					more = false;
 					break;
 				}
-				next = end - base > 32u ? base + 32u : end;
+				next = base + min(32u, end - base);
 				const uint32_t i = base + lane;
 				pending = __ballot_sync(0xffffffffu, lane < end - base && arrays.hitTriangle[i] < -1);
 				continue;
