@@ -48,9 +48,9 @@ EXTRA_LIGHTS = 64
 # converged: two 32-frame halves differ by a relative MSE of 30, which swamps the method's own error).
 REFERENCE_FRAMES = 1024
 ERROR_FRAMES = 120         # frames the relMSE and bias are averaged over
-# DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) per frame of the GI temporal pass's
-# three kernels on this workload, one launch each, captured from the current build.
-DOMINANT_TRAFFIC = {"gi_temporal": 165.4e6}
+# DRAM bytes (ncu dram__bytes_read.sum + dram__bytes_write.sum) per frame on this workload, captured from
+# the current build: the GI temporal pass's four kernels and the DI temporal pass's one, one launch each.
+DOMINANT_TRAFFIC = {"gi_temporal": 190.5e6, "di_temporal": 153.9e6}
 SIDE_STREAM_PASSES = ("shadow", "specular")
 CACHE_TRAIN_FRAMES = 60    # online training before the radiance-cache form is timed
 WORKLOAD = ("1920x1080 frame, seeded 1M-triangle city scene, GI 1/2 res + DI + specular GI + SVGF x5 + TAA + AgX "
@@ -828,9 +828,10 @@ def own_arm(args, rank: int, world: int) -> None:
     l2_gather_gbs = gather_probe(renderer)
     fetched_gbs = float(fetched_bytes[name] / seconds / 1e9) if seconds > 0 else 0.0
     share = {name: (mean_pass[i] / ms_per_frame if ms_per_frame > 0 else 0.0) for i, name in enumerate(passes)}
-    # shadow, G-buffer, DI x2, grid x2, GI temporal (3 kernels as a wavefront), GI spatial, denoiser, composite,
-    # display (auto exposure when on, then TAA + tone mapping), specular (3 kernels as a wavefront)
-    gi_temporal_kernels = 3 if settings.wavefront else 1
+    # shadow, G-buffer, DI x2, grid x2, GI temporal (4 kernels as a wavefront: candidates, rays, their
+    # re-walk, shading), GI spatial, denoiser, composite, display (auto exposure when on, then TAA +
+    # tone mapping), specular (3 kernels as a wavefront)
+    gi_temporal_kernels = 4 if settings.wavefront else 1
     launches = (2 + (2 if plan.di_active else 0) + 2 + gi_temporal_kernels + 1
                 + (1 + plan.atrous_iterations if plan.denoiser else 0) + 1
                 + ((1 + plan.exposure) if plan.display else 0)

@@ -6,7 +6,10 @@
 // Same algorithms and arithmetic as shaders/bvh.sh (slab test 32-41,
 // Moeller-Trumbore 44-71, stackless walk 140-174, nearest-first short stack
 // 216-295), so hit ids and distances are bit-identical to the CPU
-// restatement. Every node and triangle row is one 16-byte read-only load.
+// restatement. The walks of this file's first half read each row with one
+// 16-byte read-only load; the packed tests below and warptrace.cuh's read a node
+// or a triangle's first two rows with one of 32 bytes where the scene's rows
+// start on that (wideRows).
 #pragma once
 
 #include "common.cuh"

@@ -8,7 +8,9 @@
 // pixel. In the deterministic mode each cell keeps its C lowest pixel
 // indices in increasing order, by an atomicMin cascade down the cell's
 // entries (each lane carries the larger value onwards), which leaves the
-// same list whatever the arrival order. Bound by the latency of the atomics
+// same list whatever the arrival order. Which slot a cell gets depends on that
+// order, and so does, in a table so full that eight probes run out (status bit
+// 1), which cells get none. Bound by the latency of the atomics
 // of one lane, up to C in a row; the cascade starts behind the entries known
 // to be smaller (below). us after the clear, from slot 0 / behind an entry
 // found by halves / by quarters, C 32: 960x540 receivers of the 1M-triangle city
