@@ -155,6 +155,7 @@ class ClockSampler:
         self.device = device
         self.proc = None
         self.lines = []
+        self.before = 0
         self.thread = None
 
     def start(self):
@@ -166,6 +167,12 @@ class ClockSampler:
             self.thread.start()
         except (OSError, FileNotFoundError):
             self.proc = None
+            return
+        # The first sample can come later than a short timed region ends; it is of the idle GPU.
+        deadline = time.monotonic() + 3.0
+        while not self.lines and time.monotonic() < deadline:
+            time.sleep(0.01)
+        self.before = len(self.lines)
 
     def _read(self):
         for line in self.proc.stdout:
@@ -182,7 +189,7 @@ class ClockSampler:
         self.thread.join(timeout=2)
         sm, mx, reasons = [], [], set()
         names = ["hw_slowdown", "hw_thermal_slowdown", "sw_thermal_slowdown", "sw_power_cap"]
-        for line in self.lines:
+        for line in self.lines[self.before:]:
             parts = [p.strip() for p in line.split(",")]
             if len(parts) < 9:
                 continue
