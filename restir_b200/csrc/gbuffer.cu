@@ -153,7 +153,8 @@ extern "C" int restir_shadow_atlas(const RestirParams* params, const RestirScene
 	// Not split: alone its 512x512 faces gain little (10k nodes 122 us, split 126;
 	// 1.9M nodes 905 and 887), and in a frame, where it runs beside the other stream's
 	// passes, the longer code costs them: 1920x1080 in the 1M-triangle city 8.04 ms
-	// split, 7.98 not; 256x256 in the 100k-triangle city 2.29 and 2.18.
+	// split, 7.98 not; 256x256 in the 100k-triangle city 2.29 and 2.18; 440x247 in
+	// one of 259k triangles without point lights 1.34 and 1.15.
 	(wideRows(bvh) ? shadowAtlasKernel<true> : shadowAtlasKernel<false>)<<<grid, 64, 0, asStream(stream)>>>(*params, bvh, atlas);
 	return launchStatus();
 }
